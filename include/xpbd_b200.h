@@ -639,6 +639,24 @@ int xpbd_adam(int32_t rows, int32_t cols, float* w, const float* g, int32_t ld_g
 int xpbd_mse_grad(int32_t m, int32_t m_pad, int32_t n_out, int32_t ld, const float* y, int32_t ld_y, const float* t,
                   int32_t ld_t, uint16_t* d, uint16_t* d_t, int32_t ld_dt, float* loss, xpbd_stream_t stream);
 
+/* The cage network (64 -> 4 x 256 GELU -> 3) and its buffers.  BF16 weights
+ * row-major [out][in] (the last one 16 rows, rows 3.. zero) and FP32 biases;
+ * sample-major buffers have m_pad rows (a multiple of 64), transposed ones
+ * m_pad columns.  Pointers that a call does not use may be null. */
+typedef struct XpbdMlp {
+    int32_t m, m_pad;       /* samples in use, rows of the buffers */
+    const uint16_t* x;      /* [m_pad][64] features */
+    const uint16_t* w[5];
+    const float* b[5];
+    float* z[4];            /* [m_pad][256] pre-activations of the hidden layers (training) */
+    uint16_t* ht[4];        /* [256][m_pad] activations of the hidden layers, transposed (training) */
+    float* y;               /* [m_pad][16] outputs (columns 0..2 written) */
+    int32_t* status;        /* XPBD_STATUS_MMA_TIMEOUT, optional */
+} XpbdMlp;
+
+/* Forward of all m_pad rows in one launch; train != 0 also writes z and ht. */
+int xpbd_mlp_forward(const XpbdMlp* p, int32_t train, xpbd_stream_t stream);
+
 /* Static description of the cage for the feature kernel (cage order j). */
 typedef struct XpbdCageFeatures {
     int32_t n_cage, m_pad;     /* cage vertices; rows of the feature matrix (>= n_cage) */

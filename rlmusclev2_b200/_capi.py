@@ -116,6 +116,12 @@ class XpbdGemm(C.Structure):
                 ("status", C.c_void_p)]
 
 
+class XpbdMlp(C.Structure):
+    _fields_ = [("m", C.c_int32), ("m_pad", C.c_int32), ("x", C.c_void_p), ("w", C.c_void_p * 5),
+                ("b", C.c_void_p * 5), ("z", C.c_void_p * 4), ("ht", C.c_void_p * 4), ("y", C.c_void_p),
+                ("status", C.c_void_p)]
+
+
 class XpbdCageFeatures(C.Structure):
     _fields_ = [("n_cage", C.c_int32), ("m_pad", C.c_int32), ("coarse_lib", C.c_void_p), ("nbr", C.c_void_p),
                 ("owner", C.c_void_p), ("act_muscle", C.c_void_p), ("cage_bone", C.c_void_p), ("cage_w", C.c_void_p),
@@ -176,6 +182,7 @@ _SIGS = {
                    P, P, C.c_int32, P], C.c_int),
     "xpbd_mse_grad": ([C.c_int32, C.c_int32, C.c_int32, C.c_int32, P, C.c_int32, P, C.c_int32, P, P, C.c_int32, P, P],
                       C.c_int),
+    "xpbd_mlp_forward": ([C.POINTER(XpbdMlp), C.c_int32, P], C.c_int),
     "xpbd_cage_features": ([C.POINTER(XpbdCageFeatures), P, P, P, P, P], C.c_int),
     "xpbd_cage_apply": ([C.c_int32, P, P, P, C.c_int32, C.c_float, P, P], C.c_int),
     "xpbd_cage_target": ([C.c_int32, P, P, P, C.c_float, P, P], C.c_int),

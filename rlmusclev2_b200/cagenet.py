@@ -96,7 +96,6 @@ class CageMLP:
         self.X = torch.zeros((M, 64), dtype=bf, device=dev)
         self.Xt = torch.zeros((64, M), dtype=bf, device=dev)
         self.Z = [torch.zeros((M, 256), dtype=f32, device=dev) for _ in range(4)]
-        self.H = [None] + [torch.zeros((M, 256), dtype=bf, device=dev) for _ in range(4)]
         self.Ht = [self.Xt] + [torch.zeros((256, M), dtype=bf, device=dev) for _ in range(4)]
         self.Y = torch.zeros((M, OUT_PAD_FWD), dtype=f32, device=dev)
         self.dY = torch.zeros((M, OUT_PAD_BWD), dtype=bf, device=dev)
@@ -131,22 +130,25 @@ class CageMLP:
 
     # ------------------------------------------------------------ forward
     def forward(self, m: int, train: bool = True) -> torch.Tensor:
-        """Forward of the first m rows of X (Xt must hold X's transpose when a
-        backward follows).  train=False stores only what the next layer reads
-        (no pre-activations, no transposed copies) and splits each layer over
-        four 64-column tiles.  Returns Y[:m, :3] (a view)."""
-        lib, sp = self.lib, self._sp
-        H = [self.X] + self.H[1:]
-        for l in range(4):
-            if train:
-                gemm(lib, sp, H[l], self.Wb[l], self.m_pad, 256, DIMS[l], bias=self.b[l], act=1, out_pre=self.Z[l],
-                     out_bf16=self.H[l + 1], out_bf16_t=self.Ht[l + 1], status=self.status)
-            else:
-                gemm(lib, sp, H[l], self.Wb[l], self.m_pad, 256, DIMS[l], bias=self.b[l], act=1,
-                     out_bf16=self.H[l + 1], status=self.status, n_tile=64)
-        gemm(lib, sp, self.H[4], self.Wb[4], self.m_pad, 3, 256, bias=self.bpad4, act=0, out_f32=self.Y,
-             status=self.status, n_tile=16)
+        """Forward of the first m rows of X in one launch (Xt must hold X's
+        transpose when a backward follows).  train=False writes only the
+        outputs (no pre-activations, no transposed activations).  Returns
+        Y[:m, :3] (a view)."""
+        p = self._mlp(m)
+        if train:
+            p.z[:] = [t.data_ptr() for t in self.Z]
+            p.ht[:] = [t.data_ptr() for t in self.Ht[1:]]
+        capi.check(self.lib.xpbd_mlp_forward(C.byref(p), int(train), self._sp))
         return self.Y[:m, :3]
+
+    def _mlp(self, m: int) -> capi.XpbdMlp:
+        """The library's view of the network's inference buffers."""
+        p = capi.XpbdMlp()
+        p.m, p.m_pad = int(m), self.m_pad
+        p.x, p.y, p.status = self.X.data_ptr(), self.Y.data_ptr(), self.status.data_ptr()
+        p.w[:] = [t.data_ptr() for t in self.Wb]
+        p.b[:] = [t.data_ptr() for t in self.b]
+        return p
 
     # ----------------------------------------------------------- backward
     def backward(self, m: int, target: torch.Tensor) -> None:

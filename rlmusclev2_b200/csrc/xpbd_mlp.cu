@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include "xpbd_common.cuh"
+#include "xpbd_mma.cuh"
 
 using namespace xpbd;
 
@@ -36,13 +37,8 @@ constexpr int kThreads = 128;
 constexpr int kKB = 64;                 // k per stage
 constexpr uint32_t kLbo = 128;          // bytes between the two 8-wide k halves of a core-matrix pair
 constexpr uint32_t kSbo = 1024;         // bytes between 8-row groups (8 k-chunks x 128 B)
-constexpr long kWaitLimit = 1L << 22;   // try_wait polls (each suspends briefly): well over a second
 
 __device__ __forceinline__ bool aligned_ptr16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // Byte offset of element (r, k) of a 64-wide k block in the canonical layout.
 __device__ __forceinline__ uint32_t kmajor_off(int r, int k) {
@@ -56,53 +52,6 @@ __device__ __forceinline__ uint64_t smem_desc_lbo_sbo(uint32_t addr, uint32_t lb
            (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
 }
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) { return smem_desc_lbo_sbo(addr, kLbo, kSbo); }
-
-// Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D, M = 128.
-__host__ __device__ constexpr uint32_t instr_desc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
-    for (long i = 0; i < kWaitLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-
-// tanh(u) = 1 - 2 / (exp(2u) + 1) with the fast exponential (relative error
-// ~1e-6, far below the BF16 rounding of the activations it feeds); the
-// clamp keeps exp finite.
-__device__ __forceinline__ float tanh_fast(float u) {
-    const float e = __expf(2.f * fminf(fmaxf(u, -15.f), 15.f));
-    return 1.f - __fdividef(2.f, e + 1.f);
-}
-__device__ __forceinline__ float gelu_f(float x) {
-    const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-    return 0.5f * x * (1.f + tanh_fast(u));
-}
-__device__ __forceinline__ float gelu_grad_f(float x) {
-    const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-    const float t = tanh_fast(u);
-    return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 // Copy a (rows x 64) k block (rows valid of nrows_valid, zero beyond) into
 // the canonical layout at smem byte address base.
@@ -289,18 +238,6 @@ constexpr int kTmaStages = 4;
 // alternate 16-column chunks.
 constexpr int kTmaThreads = 256;
 
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
-            dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
 __global__ void __launch_bounds__(kTmaThreads, 1)
     k_gemm_bf16_tma(const __grid_constant__ XpbdGemm G, const __grid_constant__ CUtensorMap ta,
                     const __grid_constant__ CUtensorMap tb, int n_tile, int tmem_cols) {
@@ -465,23 +402,6 @@ __global__ void k_mse_grad(int m, int m_pad, int n_out, int ld, const float* __r
     const __nv_bfloat16 h = __float2bfloat16_rn(gval);
     reinterpret_cast<__nv_bfloat16*>(d)[i] = h;
     if (dt) reinterpret_cast<__nv_bfloat16*>(dt)[size_t(c) * ld_dt + r] = h;
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against the driver library); null when the driver does not provide it.
-PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        cudaGetLastError();
-    }
-    return fn;
 }
 
 // Tensor map of a K-major BF16 operand [rows][ld] (k < ld used): boxes of

@@ -155,3 +155,36 @@ def test_gemm_tma_operands_equal_thread_staged(m, n, k):
     assert torch.isfinite(y).all()
     gl = 0.5 * ref * (1 + torch.tanh(0.7978845608028654 * (ref + 0.044715 * ref ** 3)))
     assert ((y - gl).abs().max() / gl.abs().max()).item() < 1e-4
+
+
+@pytest.mark.parametrize("m", [1, 64, 65, 300, 9425, 9600])
+@pytest.mark.parametrize("train", [False, True])
+def test_fused_forward_equals_layer_gemms(m, train):
+    """The one-launch forward against one xpbd_gemm_bf16 per layer: the same
+    MMAs in the same k order and the same epilogue arithmetic, so outputs,
+    pre-activations and transposed activations are equal bit for bit."""
+    import ctypes as C
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(m)
+    net = CageMLP(dev, m, seed=m)
+    for l in range(5):
+        net.b[l].copy_(0.1 * torch.randn(DIMS[l + 1], device=dev, generator=g))
+    net.refresh_copies()
+    net.X[:m].copy_(torch.randn((m, 64), device=dev, generator=g).to(torch.bfloat16))
+    y = net.forward(m, train=train).clone()
+    M = net.m_pad
+    lib, sp = _lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    h = net.X
+    for l in range(4):
+        z = torch.zeros((M, 256), device=dev)
+        hn, ht = (torch.zeros(s, dtype=torch.bfloat16, device=dev) for s in ((M, 256), (256, M)))
+        gemm(lib, sp, h, net.Wb[l], M, 256, DIMS[l], bias=net.b[l], act=1, out_pre=z, out_bf16=hn, out_bf16_t=ht)
+        if train:
+            assert torch.equal(net.Z[l], z), l
+            assert torch.equal(net.Ht[l + 1], ht), l
+        h = hn
+    ref = torch.zeros((M, 16), device=dev)
+    gemm(lib, sp, h, net.Wb[4], M, 3, 256, bias=net.bpad4, out_f32=ref, n_tile=16)
+    torch.cuda.synchronize()
+    assert int(net.status.item()) == 0
+    assert torch.equal(y, ref[:m, :3])
