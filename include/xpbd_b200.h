@@ -633,6 +633,20 @@ int xpbd_adam(int32_t rows, int32_t cols, float* w, const float* g, int32_t ld_g
               float beta1, float beta2, float eps, int32_t step, uint16_t* w_bf16, uint16_t* w_bf16_t, int32_t ld_t,
               xpbd_stream_t stream);
 
+/* The same step on up to XPBD_ADAM_MAX_ITEMS tensors in one launch. */
+#define XPBD_ADAM_MAX_ITEMS 16
+typedef struct XpbdAdamItem {
+    int32_t rows, cols, ld_g, ld_t;
+    float* w;
+    const float* g;
+    float* m1;
+    float* m2;
+    uint16_t* w_bf16;
+    uint16_t* w_bf16_t;
+} XpbdAdamItem;
+int xpbd_adam_multi(int32_t n, const XpbdAdamItem* items, float lr, float beta1, float beta2, float eps, int32_t step,
+                    xpbd_stream_t stream);
+
 /* Mean-squared-error gradient 2 (y - t) / (m n_out) of the valid m x n_out
  * block into the BF16 (m_pad x ld) buffer d (zero elsewhere) and optionally
  * its transpose d_t[ld][ld_dt]; loss[0] += sum (y - t)^2. */
@@ -652,10 +666,23 @@ typedef struct XpbdMlp {
     uint16_t* ht[4];        /* [256][m_pad] activations of the hidden layers, transposed (training) */
     float* y;               /* [m_pad][16] outputs (columns 0..2 written) */
     int32_t* status;        /* XPBD_STATUS_MMA_TIMEOUT, optional */
+    /* backward only */
+    const uint16_t* xt;     /* [64][m_pad] features, transposed */
+    const uint16_t* wt[5];  /* weights transposed [in][out]; wt[4] is [256][64], columns 3.. zero; wt[0] unused */
+    const float* target;    /* [m][3] */
+    uint16_t* dzt[4];       /* [256][m_pad] deltas of the hidden layers, transposed (written) */
+    uint16_t* dyt;          /* [3][m_pad] loss gradient at the outputs, transposed (written) */
+    float* gw[5];           /* weight gradients [out][in] */
+    float* gb[5];           /* bias gradients */
+    float* loss;            /* += sum of squared errors */
 } XpbdMlp;
 
 /* Forward of all m_pad rows in one launch; train != 0 also writes z and ht. */
 int xpbd_mlp_forward(const XpbdMlp* p, int32_t train, xpbd_stream_t stream);
+
+/* Gradients of the mean squared error of y[:m, :3] against target, after
+ * xpbd_mlp_forward with train: two launches. */
+int xpbd_mlp_backward(const XpbdMlp* p, xpbd_stream_t stream);
 
 /* Static description of the cage for the feature kernel (cage order j). */
 typedef struct XpbdCageFeatures {

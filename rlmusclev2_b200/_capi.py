@@ -119,7 +119,15 @@ class XpbdGemm(C.Structure):
 class XpbdMlp(C.Structure):
     _fields_ = [("m", C.c_int32), ("m_pad", C.c_int32), ("x", C.c_void_p), ("w", C.c_void_p * 5),
                 ("b", C.c_void_p * 5), ("z", C.c_void_p * 4), ("ht", C.c_void_p * 4), ("y", C.c_void_p),
-                ("status", C.c_void_p)]
+                ("status", C.c_void_p), ("xt", C.c_void_p), ("wt", C.c_void_p * 5), ("target", C.c_void_p),
+                ("dzt", C.c_void_p * 4), ("dyt", C.c_void_p), ("gw", C.c_void_p * 5), ("gb", C.c_void_p * 5),
+                ("loss", C.c_void_p)]
+
+
+class XpbdAdamItem(C.Structure):
+    _fields_ = [("rows", C.c_int32), ("cols", C.c_int32), ("ld_g", C.c_int32), ("ld_t", C.c_int32),
+                ("w", C.c_void_p), ("g", C.c_void_p), ("m1", C.c_void_p), ("m2", C.c_void_p),
+                ("w_bf16", C.c_void_p), ("w_bf16_t", C.c_void_p)]
 
 
 class XpbdCageFeatures(C.Structure):
@@ -183,6 +191,9 @@ _SIGS = {
     "xpbd_mse_grad": ([C.c_int32, C.c_int32, C.c_int32, C.c_int32, P, C.c_int32, P, C.c_int32, P, P, C.c_int32, P, P],
                       C.c_int),
     "xpbd_mlp_forward": ([C.POINTER(XpbdMlp), C.c_int32, P], C.c_int),
+    "xpbd_mlp_backward": ([C.POINTER(XpbdMlp), P], C.c_int),
+    "xpbd_adam_multi": ([C.c_int32, C.POINTER(XpbdAdamItem), C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, P],
+                        C.c_int),
     "xpbd_cage_features": ([C.POINTER(XpbdCageFeatures), P, P, P, P, P], C.c_int),
     "xpbd_cage_apply": ([C.c_int32, P, P, P, C.c_int32, C.c_float, P, P], C.c_int),
     "xpbd_cage_target": ([C.c_int32, P, P, P, C.c_float, P, P], C.c_int),

@@ -1,5 +1,5 @@
 """Per-cage-vertex MLP of the learned coarse correction, on the library's
-tensor-core kernels (xpbd_gemm_bf16 and friends).
+tensor-core kernels (xpbd_mlp_forward, xpbd_mlp_backward, xpbd_adam_multi).
 
 Network: 64 features -> 4 hidden layers of width 256 with GELU -> 3 outputs
 (the cage correction in millimetres).  Weights live as FP32 masters with BF16
@@ -90,7 +90,6 @@ class CageMLP:
                 lst.append(torch.zeros((fo, fi), dtype=f32, device=dev))
             for lst in (self.mb, self.vb):
                 lst.append(torch.zeros(fo, dtype=f32, device=dev))
-        self.bpad4 = torch.zeros(OUT_PAD_FWD, dtype=f32, device=dev)
         self.refresh_copies()
         M = self.m_pad
         self.X = torch.zeros((M, 64), dtype=bf, device=dev)
@@ -98,10 +97,8 @@ class CageMLP:
         self.Z = [torch.zeros((M, 256), dtype=f32, device=dev) for _ in range(4)]
         self.Ht = [self.Xt] + [torch.zeros((256, M), dtype=bf, device=dev) for _ in range(4)]
         self.Y = torch.zeros((M, OUT_PAD_FWD), dtype=f32, device=dev)
-        self.dY = torch.zeros((M, OUT_PAD_BWD), dtype=bf, device=dev)
-        self.dYt = torch.zeros((OUT_PAD_BWD, M), dtype=bf, device=dev)
-        self.dZ = [torch.zeros((M, 256), dtype=bf, device=dev) for _ in range(2)]
-        self.dZt = [torch.zeros((256, M), dtype=bf, device=dev) for _ in range(2)]
+        self.dYt = torch.zeros((DIMS[-1], M), dtype=bf, device=dev)
+        self.dZt = [torch.zeros((256, M), dtype=bf, device=dev) for _ in range(4)]
         self.gW = [torch.zeros((DIMS[l + 1], DIMS[l]), dtype=f32, device=dev) for l in range(5)]
         self.gb = [torch.zeros(DIMS[l + 1], dtype=f32, device=dev) for l in range(5)]
         self.loss = torch.zeros(1, dtype=f32, device=dev)
@@ -115,7 +112,6 @@ class CageMLP:
                 fo = DIMS[l + 1]
                 self.Wb[l][:fo].copy_(self.W[l].to(torch.bfloat16))
                 self.Wt[l][:, :fo].copy_(self.W[l].t().to(torch.bfloat16))
-            self.bpad4[:3].copy_(self.b[4])
 
     def state_dict(self) -> dict:
         return {f"W{l}": self.W[l].cpu().numpy() for l in range(5)} | {f"b{l}": self.b[l].cpu().numpy()
@@ -153,36 +149,26 @@ class CageMLP:
     # ----------------------------------------------------------- backward
     def backward(self, m: int, target: torch.Tensor) -> None:
         """Gradients of the mean squared error of Y[:m, :3] against target
-        (m x 3, FP32) into gW, gb; adds sum of squared errors to loss."""
-        lib, sp, M = self.lib, self._sp, self.m_pad
+        (m x 3, FP32) into gW, gb, in two launches; adds the sum of squared
+        errors to loss."""
         tgt = target.contiguous()
-        capi.check(lib.xpbd_mse_grad(int(m), M, 3, OUT_PAD_BWD, _p(self.Y), OUT_PAD_FWD, _p(tgt), 3, _p(self.dY),
-                                     _p(self.dYt), M, _p(self.loss), sp))
-        # last layer
-        gemm(lib, sp, self.dYt, self.Ht[4], 3, 256, M, out_f32=self.gW[4], status=self.status)
-        capi.check(lib.xpbd_colsum_bf16(3, int(m), _p(self.dYt), M, _p(self.gb[4]), sp))
-        gemm(lib, sp, self.dY, self.Wt[4], M, 256, OUT_PAD_BWD, gelu_grad_of=self.Z[3], out_bf16=self.dZ[0],
-             out_bf16_t=self.dZt[0], status=self.status)
-        cur = 0
-        for l in range(3, -1, -1):
-            gemm(lib, sp, self.dZt[cur], self.Ht[l], 256, DIMS[l], M, out_f32=self.gW[l], status=self.status)
-            capi.check(lib.xpbd_colsum_bf16(256, int(m), _p(self.dZt[cur]), M, _p(self.gb[l]), sp))
-            if l > 0:
-                nxt = 1 - cur
-                gemm(lib, sp, self.dZ[cur], self.Wt[l], M, 256, 256, gelu_grad_of=self.Z[l - 1],
-                     out_bf16=self.dZ[nxt], out_bf16_t=self.dZt[nxt], status=self.status)
-                cur = nxt
+        p = self._mlp(m)
+        p.z[:] = [t.data_ptr() for t in self.Z]
+        p.ht[:] = [t.data_ptr() for t in self.Ht[1:]]
+        p.xt, p.target, p.dyt, p.loss = (t.data_ptr() for t in (self.Xt, tgt, self.dYt, self.loss))
+        p.wt[:] = [t.data_ptr() for t in self.Wt]
+        p.dzt[:] = [t.data_ptr() for t in self.dZt]
+        p.gw[:] = [t.data_ptr() for t in self.gW]
+        p.gb[:] = [t.data_ptr() for t in self.gb]
+        capi.check(self.lib.xpbd_mlp_backward(C.byref(p), self._sp))
 
     def adam_step(self, lr: float = 1e-3, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8) -> None:
         self.step_count += 1
-        lib, sp, t = self.lib, self._sp, self.step_count
+        items = (capi.XpbdAdamItem * 10)()
         for l in range(5):
             fo, fi = DIMS[l + 1], DIMS[l]
-            capi.check(lib.xpbd_adam(fo, fi, _p(self.W[l]), _p(self.gW[l]), fi, _p(self.mW[l]), _p(self.vW[l]),
-                                     C.c_float(lr), C.c_float(beta1), C.c_float(beta2), C.c_float(eps), t,
-                                     _p(self.Wb[l]), _p(self.Wt[l]), self.Wt[l].shape[1], sp))
-            capi.check(lib.xpbd_adam(1, fo, _p(self.b[l]), _p(self.gb[l]), fo, _p(self.mb[l]), _p(self.vb[l]),
-                                     C.c_float(lr), C.c_float(beta1), C.c_float(beta2), C.c_float(eps), t, None, None,
-                                     1, sp))
-        with torch.cuda.stream(self.stream):
-            self.bpad4[:3].copy_(self.b[4])
+            items[2 * l] = (fo, fi, fi, self.Wt[l].shape[1], self.W[l].data_ptr(), self.gW[l].data_ptr(),
+                            self.mW[l].data_ptr(), self.vW[l].data_ptr(), self.Wb[l].data_ptr(), self.Wt[l].data_ptr())
+            items[2 * l + 1] = (1, fo, fo, 1, self.b[l].data_ptr(), self.gb[l].data_ptr(), self.mb[l].data_ptr(),
+                                self.vb[l].data_ptr(), None, None)
+        capi.check(self.lib.xpbd_adam_multi(10, items, lr, beta1, beta2, eps, self.step_count, self._sp))

@@ -366,22 +366,35 @@ __global__ void k_colsum_bf16(int n_out, int m, const uint16_t* __restrict__ dzt
 
 // Adam on FP32 master weights (Kingma & Ba 2015), with the BF16 copy and the
 // BF16 transposed copy (rows x cols -> cols x ld_t) refreshed in place.
-__global__ void k_adam(int rows, int cols, float* __restrict__ w, const float* __restrict__ g, int ld_g,
-                       float* __restrict__ m1, float* __restrict__ m2, float lr, float b1, float b2, float eps,
-                       float c1, float c2, uint16_t* __restrict__ wb, uint16_t* __restrict__ wt, int ld_t) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    const int r = i / cols, c = i % cols;
-    const float gi = g[size_t(r) * ld_g + c];
-    const float a = b1 * m1[i] + (1.f - b1) * gi;
-    const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    const float wi = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-    w[i] = wi;
+__device__ __forceinline__ void adam_element(const XpbdAdamItem& t, int i, float lr, float b1, float b2, float eps,
+                                             float c1, float c2) {
+    const int r = i / t.cols, c = i % t.cols;
+    const float gi = t.g[size_t(r) * t.ld_g + c];
+    const float a = b1 * t.m1[i] + (1.f - b1) * gi;
+    const float b = b2 * t.m2[i] + (1.f - b2) * gi * gi;
+    t.m1[i] = a;
+    t.m2[i] = b;
+    const float wi = t.w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    t.w[i] = wi;
     const __nv_bfloat16 h = __float2bfloat16_rn(wi);
-    if (wb) reinterpret_cast<__nv_bfloat16*>(wb)[i] = h;
-    if (wt) reinterpret_cast<__nv_bfloat16*>(wt)[size_t(c) * ld_t + r] = h;
+    if (t.w_bf16) reinterpret_cast<__nv_bfloat16*>(t.w_bf16)[i] = h;
+    if (t.w_bf16_t) reinterpret_cast<__nv_bfloat16*>(t.w_bf16_t)[size_t(c) * t.ld_t + r] = h;
+}
+
+// All tensors of a step in one launch (ten launches of 3-4 us each before, a
+// quarter of them one CTA): item k owns blocks [first[k], first[k + 1]).
+struct AdamItems {
+    XpbdAdamItem t[XPBD_ADAM_MAX_ITEMS];
+    int first[XPBD_ADAM_MAX_ITEMS + 1];
+    int n;
+};
+
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamItems A, float lr, float b1, float b2,
+                                              float eps, float c1, float c2) {
+    int k = 0;
+    while (k + 1 < A.n && int(blockIdx.x) >= A.first[k + 1]) ++k;
+    const int i = (int(blockIdx.x) - A.first[k]) * 256 + int(threadIdx.x);
+    if (i < A.t[k].rows * A.t[k].cols) adam_element(A.t[k], i, lr, b1, b2, eps, c1, c2);
 }
 
 // Loss gradient of the mean squared error over the valid rows:
@@ -463,16 +476,33 @@ int xpbd_colsum_bf16(int32_t n_out, int32_t m, const uint16_t* dzt, int32_t ld, 
     return cuda_check("xpbd_colsum_bf16");
 }
 
+int xpbd_adam_multi(int32_t n, const XpbdAdamItem* items, float lr, float beta1, float beta2, float eps, int32_t step,
+                    xpbd_stream_t stream) {
+    if (n < 1 || n > XPBD_ADAM_MAX_ITEMS || !items || step < 1)
+        return fail(XPBD_ERR_ARG, "xpbd_adam_multi: 1..16 items, step >= 1");
+    AdamItems A;
+    A.n = n;
+    A.first[0] = 0;
+    for (int k = 0; k < n; ++k) {
+        const XpbdAdamItem& t = items[k];
+        if (t.rows <= 0 || t.cols <= 0 || !t.w || !t.g || !t.m1 || !t.m2 || t.ld_g < t.cols ||
+            (t.w_bf16_t && t.ld_t < t.rows))
+            return fail(XPBD_ERR_ARG, "xpbd_adam_multi: bad item");
+        A.t[k] = t;
+        A.first[k + 1] = A.first[k] + (t.rows * t.cols + 255) / 256;
+    }
+    const float c1 = 1.f - powf(beta1, float(step)), c2 = 1.f - powf(beta2, float(step));
+    k_adam<<<A.first[n], 256, 0, (cudaStream_t)stream>>>(A, lr, beta1, beta2, eps, c1, c2);
+    return cuda_check("xpbd_adam_multi");
+}
+
 int xpbd_adam(int32_t rows, int32_t cols, float* w, const float* g, int32_t ld_g, float* m1, float* m2, float lr,
               float beta1, float beta2, float eps, int32_t step, uint16_t* w_bf16, uint16_t* w_bf16_t, int32_t ld_t,
               xpbd_stream_t stream) {
     if (rows <= 0 || cols <= 0 || !w || !g || !m1 || !m2 || step < 1 || ld_g < cols || (w_bf16_t && ld_t < rows))
         return fail(XPBD_ERR_ARG, "xpbd_adam: bad arguments");
-    const float c1 = 1.f - powf(beta1, float(step)), c2 = 1.f - powf(beta2, float(step));
-    const int n = rows * cols;
-    k_adam<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(rows, cols, w, g, ld_g, m1, m2, lr, beta1, beta2, eps,
-                                                              c1, c2, w_bf16, w_bf16_t, ld_t);
-    return cuda_check("xpbd_adam");
+    const XpbdAdamItem t = {rows, cols, ld_g, ld_t, w, g, m1, m2, w_bf16, w_bf16_t};
+    return xpbd_adam_multi(1, &t, lr, beta1, beta2, eps, step, stream);
 }
 
 int xpbd_mse_grad(int32_t m, int32_t m_pad, int32_t n_out, int32_t ld, const float* y, int32_t ld_y, const float* t,

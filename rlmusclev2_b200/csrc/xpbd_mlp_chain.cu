@@ -91,28 +91,40 @@ __device__ __forceinline__ uint32_t a_off(int row, int k) {
 }
 
 // A layer's activations, transposed, to global memory: out[col][ld] for the
-// CTA's 64 samples.  A lane reads 8 columns of one sample (16 bytes, swizzled:
-// no conflicts) and a warp's stores cover 32 consecutive samples of a column.
+// CTA's 64 samples.  A lane reads 8 columns of two neighbouring samples (16
+// swizzled bytes each) and stores pairs: one full 128-byte line per column.
 __device__ __forceinline__ void store_transposed(const unsigned char* sa, uint16_t* out, int ld, int m0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int u = warp; u < 2 * (kHid / 8); u += kChainThreads / 32) {
-        const int j = (u & 1) * 32 + lane, c0 = (u >> 1) * 8;  // sample in the CTA, first column
-        const uint4 q = *reinterpret_cast<const uint4*>(sa + a_off((j >> 4) * 32 + (j & 15), c0));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    const int j = 2 * lane, row = (j >> 4) * 32 + (j & 15);
+    for (int u = warp; u < kHid / 8; u += kChainThreads / 32) {
+        const int c0 = 8 * u;
+        const uint4 a = *reinterpret_cast<const uint4*>(sa + a_off(row, c0));
+        const uint4 b = *reinterpret_cast<const uint4*>(sa + a_off(row + 1, c0));
+        const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            out[size_t(c0 + e) * ld + m0 + j] = uint16_t(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
+            *reinterpret_cast<uint32_t*>(out + size_t(c0 + e) * ld + m0 + j) =
+                __byte_perm(wa[e >> 1], wb[e >> 1], e & 1 ? 0x7632 : 0x5410);
     }
 }
 
-template <bool TRAIN>
+// INFER: outputs only.  TRAIN: also the hidden layers' pre-activations and
+// transposed activations.  BACK: the deltas of the hidden layers from the
+// loss gradient at the outputs, dZ_{l-1} = (dZ_l W_l) gelu'(Z_{l-1}): the same
+// chain with the transposed weights (last layer first), four layers long; the
+// first A operand is the loss gradient itself, formed here from y and target.
+enum { INFER, TRAIN, BACK };
+
+template <int MODE>
 __global__ void __launch_bounds__(kChainThreads, 1)
-    k_mlp_forward(const __grid_constant__ XpbdMlp P, const __grid_constant__ ChainMaps M) {
+    k_mlp_chain(const __grid_constant__ XpbdMlp P, const __grid_constant__ ChainMaps M) {
+    constexpr int kLayers = MODE == BACK ? 4 : 5;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t s_x, s_w[4], s_acc;
     __shared__ uint32_t s_tmem;
     __shared__ int s_ok;
-    __shared__ __align__(16) float s_bias[4 * kHid + 16];
+    __shared__ __align__(16) float s_bias[MODE == BACK ? 4 : 4 * kHid + 16];
+    __shared__ float s_loss;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzle atoms are 1024 bytes
     unsigned char* sa = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t aw = base, ww = base + 4 * kABlock;
@@ -129,9 +141,12 @@ __global__ void __launch_bounds__(kChainThreads, 1)
         for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s_w[i])));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         s_ok = 1;
+        s_loss = 0.f;
     }
-    for (int i = threadIdx.x; i < 4 * kHid + 16; i += kChainThreads)
-        s_bias[i] = i < 4 * kHid ? P.b[i >> 8][i & 255] : (i - 4 * kHid < 3 ? P.b[4][i - 4 * kHid] : 0.f);
+    if constexpr (MODE != BACK) {
+        for (int i = threadIdx.x; i < 4 * kHid + 16; i += kChainThreads)
+            s_bias[i] = i < 4 * kHid ? P.b[i >> 8][i & 255] : (i - 4 * kHid < 3 ? P.b[4][i - 4 * kHid] : 0.f);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -146,17 +161,48 @@ __global__ void __launch_bounds__(kChainThreads, 1)
         }
     };
     if (threadIdx.x == 0) {
-        mbar_expect_tx(smem_u32(&s_x), kRows * 128);
-        for (int q = 0; q < 4; ++q) tma_load_2d(aw + uint32_t(q) * 32u * 128u, &M.x, 0, m0 + 16 * q, smem_u32(&s_x));
+        if constexpr (MODE != BACK) {
+            mbar_expect_tx(smem_u32(&s_x), kRows * 128);
+            for (int q = 0; q < 4; ++q) tma_load_2d(aw + uint32_t(q) * 32u * 128u, &M.x, 0, m0 + 16 * q, smem_u32(&s_x));
+        }
         load_weights(0);
+    }
+    if constexpr (MODE == BACK) {
+        // 2 (y - t) / (3 m) of the valid samples in columns 0..2, zero elsewhere;
+        // eight threads per sample, one 16-byte chunk each
+        const int j = threadIdx.x >> 3, chunk = threadIdx.x & 7, r = m0 + j;
+        uint4 d = make_uint4(0u, 0u, 0u, 0u);
+        float e2 = 0.f;
+        if (chunk == 0) {
+            float g[3] = {0.f, 0.f, 0.f};
+            if (r < P.m) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const float e = P.y[size_t(r) * 16 + c] - P.target[size_t(r) * 3 + c];
+                    g[c] = 2.f * e / float(P.m * 3);
+                    e2 += e * e;
+                }
+            }
+            d.x = pack_bf16(g[0], g[1]);
+            d.y = pack_bf16(g[2], 0.f);
+            P.dyt[r] = uint16_t(d.x & 0xffffu);
+            P.dyt[size_t(P.m_pad) + r] = uint16_t(d.x >> 16);
+            P.dyt[size_t(2 * P.m_pad) + r] = uint16_t(d.y & 0xffffu);
+        }
+        *reinterpret_cast<uint4*>(sa + a_off((j >> 4) * 32 + (j & 15), 8 * chunk)) = d;
+        for (int k = 16; k > 0; k >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, k);
+        if (lane == 0) atomicAdd(&s_loss, e2);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x == 0) atomicAdd(P.loss, s_loss);
     }
     int loaded = 0;  // last layer whose weights were asked for (thread 0)
     bool ok = true;
-    for (int l = 0; l < 5; ++l) {
+    for (int l = 0; l < kLayers; ++l) {
         const int nkb = l == 0 ? 1 : 4;
         const int n = l == 4 ? 16 : kHid;
         if (threadIdx.x == 32) {
-            bool up = l > 0 || mbar_wait(smem_u32(&s_x), 0);
+            bool up = MODE == BACK || l > 0 || mbar_wait(smem_u32(&s_x), 0);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             for (int kb = 0; kb < nkb && up; ++kb) {
                 // slot 0 is used by every layer, the others from layer 1 on
@@ -172,7 +218,7 @@ __global__ void __launch_bounds__(kChainThreads, 1)
         __syncwarp();
         if (!mbar_wait(smem_u32(&s_acc), uint32_t(l & 1))) s_ok = 0;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        if (threadIdx.x == 0 && l < 4) {  // the MMAs have read every slot: the next layer's weights may land
+        if (threadIdx.x == 0 && l + 1 < kLayers) {  // the MMAs have read every slot: the next layer's weights may land
             loaded = l + 1;
             load_weights(l + 1);
         }
@@ -180,7 +226,6 @@ __global__ void __launch_bounds__(kChainThreads, 1)
         const int q = warp & 3, cg = warp >> 2;
         const int r0 = lane >> 2, cp = 2 * (lane & 3);
         if (l < 4) {
-            const float* bias = s_bias + l * kHid;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int c0 = cg * 64 + h * 32;
@@ -189,18 +234,28 @@ __global__ void __launch_bounds__(kChainThreads, 1)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int c = c0 + 8 * i + cp;
-                    const float2 bb = *reinterpret_cast<const float2*>(bias + c);
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
                         const int r = r0 + 8 * s;
-                        const float z0 = v[4 * i + 2 * s] + bb.x, z1 = v[4 * i + 2 * s + 1] + bb.y;
-                        if (TRAIN)
-                            *reinterpret_cast<float2*>(P.z[l] + size_t(m0 + 16 * q + r) * kHid + c) = make_float2(z0, z1);
-                        *reinterpret_cast<uint32_t*>(sa + a_off(q * 32 + r, c)) = pack_bf16(gelu_f(z0), gelu_f(z1));
+                        const size_t g = size_t(m0 + 16 * q + r) * kHid + c;
+                        float y0 = v[4 * i + 2 * s], y1 = v[4 * i + 2 * s + 1];
+                        if constexpr (MODE == BACK) {
+                            const float2 z = *reinterpret_cast<const float2*>(P.z[3 - l] + g);
+                            y0 *= gelu_grad_f(z.x);
+                            y1 *= gelu_grad_f(z.y);
+                        } else {
+                            const float2 bb = *reinterpret_cast<const float2*>(s_bias + l * kHid + c);
+                            y0 += bb.x;
+                            y1 += bb.y;
+                            if (MODE == TRAIN) *reinterpret_cast<float2*>(P.z[l] + g) = make_float2(y0, y1);
+                            y0 = gelu_f(y0);
+                            y1 = gelu_f(y1);
+                        }
+                        *reinterpret_cast<uint32_t*>(sa + a_off(q * 32 + r, c)) = pack_bf16(y0, y1);
                     }
                 }
             }
-        } else if (cg == 0) {
+        } else if (MODE != BACK && cg == 0) {
             float v[16];
             tmem_ld_16x32(tmem + (uint32_t(q * 32) << 16), v);
 #pragma unroll
@@ -217,15 +272,15 @@ __global__ void __launch_bounds__(kChainThreads, 1)
         __syncthreads();
         ok = s_ok != 0;
         if (!ok) break;
-        if (TRAIN && l < 4) {
-            store_transposed(sa, P.ht[l], P.m_pad, m0);
+        if (MODE != INFER && l < 4) {
+            store_transposed(sa, MODE == BACK ? P.dzt[3 - l] : P.ht[l], P.m_pad, m0);
             __syncthreads();  // read before the next epilogue overwrites it
         }
     }
     if (!ok && threadIdx.x == 0) {
         if (P.status) atomicOr(P.status, XPBD_STATUS_MMA_TIMEOUT);
         // bounded waits for the copies in flight before the shared memory is given up
-        mbar_wait(smem_u32(&s_x), 0);
+        if (MODE != BACK) mbar_wait(smem_u32(&s_x), 0);
         for (int kb = 0; kb < (loaded == 0 ? 1 : 4); ++kb)
             mbar_wait(smem_u32(&s_w[kb]), uint32_t((kb == 0 ? loaded : loaded - 1) & 1));
     }
@@ -233,6 +288,154 @@ __global__ void __launch_bounds__(kChainThreads, 1)
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(256));
+    }
+}
+
+// Weight and bias gradients of all five layers, dW = dZ^T H over the samples
+// and db = sum of dZ, in one launch.  A tile of a 256 x 256 gradient has the
+// whole batch as its k (9,472): as GEMM launches of 2 to 8 CTAs they took
+// 131 us each, bound by the 16-byte-wide boxes that one CTA's operands came in.
+// Here 60 CTAs, one per 128 x 32 tile of any layer, stream swizzled 64-wide k
+// blocks eight deep, 50 us for all five.  The k blocks are accumulated in one
+// ascending chain in tensor memory as xpbd_gemm_bf16 does, so the sums are bit
+// for bit the same, and that chain of 592 dependent MMAs (about 160 cycles
+// each) is what bounds it: halving each CTA's operand bytes (112 CTAs of 64
+// rows) changed nothing.  A split over k is faster (25 us) and ten times
+// closer to the 64-bit sums, but then differs from the chain by 2.5e-4 of the
+// gradient's norm.  The other CTAs, on the SMs the tiles leave free, sum the
+// rows of dZ^T and dY^T.
+constexpr int kGradStages = 8;
+constexpr int kGradThreads = 256;
+constexpr int kGradM = 128, kGradN = 32;
+constexpr int kGradTiles = 3 * 16 + 4 + 8;
+constexpr uint32_t kGradStage = (kGradM + kGradN) * 128;  // A and B rows of one k block
+constexpr size_t kGradSmem = kGradStages * kGradStage + 1024;
+constexpr int kSumRows = 4 * kHid + 3;                 // rows of dZ^T and dY^T, one warp each
+constexpr int kSumCtas = (kSumRows + kGradThreads / 32 - 1) / (kGradThreads / 32);
+
+struct GradMaps {
+    CUtensorMap a[5];  // dZ^T of layers 0..3 and dY^T: [rows][m_pad], boxes 64 x 128
+    CUtensorMap b[5];  // X^T and H^T of layers 0..3, boxes 64 x 32
+};
+
+// db of one row, in xpbd_colsum_bf16's order (lane i adds elements i, i + 32,
+// ... of the m samples, then the lanes); 16 loads in flight hide their latency.
+__device__ __forceinline__ void row_sum(const XpbdMlp& P, int row) {
+    const int lane = threadIdx.x & 31;
+    if (row >= kSumRows) return;
+    const int l = row >> 8, r = row & 255;  // l = 4: dY^T
+    const uint16_t* src = (l == 4 ? P.dyt : P.dzt[l]) + size_t(r) * P.m_pad;
+    float s = 0.f;
+    int i = lane;
+    for (; i + 15 * 32 < P.m; i += 16 * 32) {
+        uint16_t v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = src[i + 32 * k];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += __uint_as_float(uint32_t(v[k]) << 16);
+    }
+    for (; i < P.m; i += 32) s += __uint_as_float(uint32_t(src[i]) << 16);
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (lane == 0) P.gb[l][r] = s;
+}
+
+__global__ void __launch_bounds__(kGradThreads, 1)
+    k_mlp_wgrad(const __grid_constant__ XpbdMlp P, const __grid_constant__ GradMaps M) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t s_full[kGradStages], s_free[kGradStages], s_acc;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_ok;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = int(blockIdx.x);
+    if (tile >= kGradTiles) {
+        row_sum(P, (tile - kGradTiles) * (kGradThreads / 32) + warp);
+        return;
+    }
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    // tiles 0..47: the 256 x 256 layers, 16 each; 48..51: layer 0 (256 x 64); 52..59: the output layer (3 x 256)
+    int l, mi, ni;
+    if (tile < 48) {
+        l = 1 + tile / 16;
+        mi = (tile >> 3) & 1;
+        ni = tile & 7;
+    } else {
+        l = tile < 52 ? 0 : 4;
+        mi = tile < 52 ? (tile >> 1) & 1 : 0;
+        ni = tile < 52 ? tile & 1 : tile - 52;
+    }
+    const int rows = l == 4 ? 3 : kHid, ldw = l == 0 ? 64 : kHid, nkb = P.m_pad / 64;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)),
+                     "r"(kGradN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    if (threadIdx.x == 32) {
+        for (int i = 0; i < kGradStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s_full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s_free[i])));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s_acc)));
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        s_ok = 1;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    if (threadIdx.x == 0) {  // copies
+        int kb = 0;
+        for (; kb < nkb; ++kb) {
+            const int st = kb % kGradStages;
+            if (kb >= kGradStages && !mbar_wait(smem_u32(&s_free[st]), uint32_t(((kb / kGradStages) - 1) & 1))) {
+                s_ok = 0;
+                break;
+            }
+            const uint32_t bar = smem_u32(&s_full[st]), sa = base + uint32_t(st) * kGradStage;
+            mbar_expect_tx(bar, kGradStage);
+            tma_load_2d(sa, &M.a[l], kb * 64, mi * kGradM, bar);
+            tma_load_2d(sa + kGradM * 128, &M.b[l], kb * 64, ni * kGradN, bar);
+        }
+        // every copy has landed before the CTA gives up its shared memory
+        for (int k = max(0, kb - kGradStages); k < kb; ++k)
+            if (!mbar_wait(smem_u32(&s_full[k % kGradStages]), uint32_t((k / kGradStages) & 1))) s_ok = 0;
+    } else if (threadIdx.x == 32) {  // MMAs
+        for (int kb = 0; kb < nkb; ++kb) {
+            const int st = kb % kGradStages;
+            if (!mbar_wait(smem_u32(&s_full[st]), uint32_t((kb / kGradStages) & 1))) {
+                s_ok = 0;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t sa = base + uint32_t(st) * kGradStage;
+            mma_block(tmem, sa, sa + kGradM * 128, instr_desc(kGradN), kb == 0);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                             smem_u32(&s_free[st]))
+                         : "memory");
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                         smem_u32(&s_acc))
+                     : "memory");
+        if (!mbar_wait(smem_u32(&s_acc), 0)) s_ok = 0;
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (s_ok) {
+        const int q = warp & 3, row = mi * kGradM + q * 32 + lane, c0 = 16 * (warp >> 2);
+        float v[16];
+        tmem_ld16(tmem + (uint32_t(q * 32) << 16) + uint32_t(c0), v);
+        if (row < rows) {
+            float4* d = reinterpret_cast<float4*>(P.gw[l] + size_t(row) * ldw + ni * kGradN + c0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+    } else if (threadIdx.x == 0 && P.status) {
+        atomicOr(P.status, XPBD_STATUS_MMA_TIMEOUT);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kGradN));
     }
 }
 
@@ -270,7 +473,8 @@ extern "C" int xpbd_mlp_forward(const XpbdMlp* p, int32_t train, xpbd_stream_t s
     }
     for (int l = 0; l < 4 && train; ++l) {
         if (!p->z[l] || !p->ht[l]) return fail(XPBD_ERR_ARG, "xpbd_mlp_forward: training needs z and ht");
-        if (!aligned16(p->z[l])) return fail(XPBD_ERR_ALIGN, "xpbd_mlp_forward: z must be 16-byte aligned");
+        if (!aligned16(p->z[l]) || !aligned16(p->ht[l]))
+            return fail(XPBD_ERR_ALIGN, "xpbd_mlp_forward: z and ht must be 16-byte aligned");
     }
     ChainMaps maps;
     bool enc = encode_sw128(&maps.x, p->x, p->m_pad, 64, 64, 16);
@@ -278,9 +482,44 @@ extern "C" int xpbd_mlp_forward(const XpbdMlp* p, int32_t train, xpbd_stream_t s
         enc = encode_sw128(&maps.w[l], p->w[l], l == 4 ? 16 : kHid, l == 0 ? 64 : kHid, l == 0 ? 64 : kHid,
                            l == 4 ? 16 : kHid);
     if (!enc) return fail(XPBD_ERR_CUDA, "xpbd_mlp_forward: tensor maps");
-    auto kern = train ? k_mlp_forward<true> : k_mlp_forward<false>;
+    auto kern = train ? k_mlp_chain<TRAIN> : k_mlp_chain<INFER>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) != cudaSuccess)
         return cuda_check("xpbd_mlp_forward: smem attribute");
     kern<<<p->m_pad / kRows, kChainThreads, kChainSmem, (cudaStream_t)stream>>>(*p, maps);
     return cuda_check("xpbd_mlp_forward");
+}
+
+extern "C" int xpbd_mlp_backward(const XpbdMlp* p, xpbd_stream_t stream) {
+    int rc;
+    if ((rc = check_mlp(p, "xpbd_mlp_backward: null argument"))) return rc;
+    if (p->m < 1 || !p->y || !p->xt || !p->target || !p->dyt || !p->loss)
+        return fail(XPBD_ERR_ARG, "xpbd_mlp_backward: m >= 1, y, xt, target, dyt and loss required");
+    if (!aligned16(p->xt) || !aligned16(p->dyt)) return fail(XPBD_ERR_ALIGN, "xpbd_mlp_backward: 16-byte alignment");
+    for (int l = 0; l < 5; ++l) {
+        if (!p->gw[l] || !p->gb[l] || (l > 0 && !p->wt[l]) || (l < 4 && (!p->z[l] || !p->ht[l] || !p->dzt[l])))
+            return fail(XPBD_ERR_ARG, "xpbd_mlp_backward: wt, z, ht, dzt, gw and gb required");
+        if (!aligned16(p->gw[l]) || !aligned16(p->wt[l]) ||
+            (l < 4 && (!aligned16(p->z[l]) || !aligned16(p->ht[l]) || !aligned16(p->dzt[l]))))
+            return fail(XPBD_ERR_ALIGN, "xpbd_mlp_backward: 16-byte alignment");
+    }
+    ChainMaps cm = {};
+    bool enc = true;
+    for (int l = 0; l < 4 && enc; ++l) {  // wt[4] (k 64), wt[3], wt[2], wt[1]
+        const int k = l == 0 ? 64 : kHid;
+        enc = encode_sw128(&cm.w[l], p->wt[4 - l], kHid, k, k, kHid);
+    }
+    GradMaps gm;
+    const int M = p->m_pad;
+    for (int l = 0; l < 5 && enc; ++l) {
+        enc = encode_sw128(&gm.a[l], l == 4 ? p->dyt : p->dzt[l], l == 4 ? 3 : kHid, M, M, kGradM);
+        enc = enc && encode_sw128(&gm.b[l], l == 0 ? p->xt : p->ht[l - 1], l == 0 ? 64 : kHid, M, M, kGradN);
+    }
+    if (!enc) return fail(XPBD_ERR_CUDA, "xpbd_mlp_backward: tensor maps");
+    if (cudaFuncSetAttribute(k_mlp_chain<BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGradSmem)) != cudaSuccess)
+        return cuda_check("xpbd_mlp_backward: smem attribute");
+    k_mlp_chain<BACK><<<M / kRows, kChainThreads, kChainSmem, (cudaStream_t)stream>>>(*p, cm);
+    k_mlp_wgrad<<<kGradTiles + kSumCtas, kGradThreads, kGradSmem, (cudaStream_t)stream>>>(*p, gm);
+    return cuda_check("xpbd_mlp_backward");
 }

@@ -184,7 +184,45 @@ def test_fused_forward_equals_layer_gemms(m, train):
             assert torch.equal(net.Ht[l + 1], ht), l
         h = hn
     ref = torch.zeros((M, 16), device=dev)
-    gemm(lib, sp, h, net.Wb[4], M, 3, 256, bias=net.bpad4, out_f32=ref, n_tile=16)
+    gemm(lib, sp, h, net.Wb[4], M, 3, 256, bias=net.b[4], out_f32=ref, n_tile=16)
     torch.cuda.synchronize()
     assert int(net.status.item()) == 0
     assert torch.equal(y, ref[:m, :3])
+
+
+@pytest.mark.parametrize("m", [1, 100, 300, 2000, 9425])
+def test_fused_backward_equals_layer_launches(m):
+    """The two-launch backward against one GEMM and one column sum per layer, in
+    the same accumulation order: deltas and gradients equal bit for bit."""
+    import ctypes as C
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(m)
+    net = CageMLP(dev, m, seed=m + 1)
+    x = torch.randn((m, 64), device=dev, generator=g).to(torch.bfloat16)
+    tgt = torch.randn((m, 3), device=dev, generator=g)
+    net.X[:m].copy_(x)
+    net.Xt[:, :m].copy_(x.t())
+    net.forward(m)
+    net.backward(m, tgt)
+    M, lib, sp = net.m_pad, _lib(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    z16 = lambda *s: torch.zeros(s, dtype=torch.bfloat16, device=dev)  # noqa: E731
+    dy, dyt, loss = z16(M, 64), z16(64, M), torch.zeros(1, device=dev)
+    capi.check(lib.xpbd_mse_grad(m, M, 3, 64, p(net.Y), 16, p(tgt), 3, p(dy), p(dyt), M, p(loss), sp))
+    assert torch.equal(net.dYt, dyt[:3])
+    assert abs(float(net.loss) - float(loss)) <= 1e-4 * float(loss)
+
+    d, dt, k = dy, dyt, 64
+    for l in range(4, -1, -1):
+        gw, gb = torch.zeros_like(net.gW[l]), torch.zeros_like(net.gb[l])
+        gemm(lib, sp, dt, net.Ht[l], DIMS[l + 1], DIMS[l], M, out_f32=gw)
+        capi.check(lib.xpbd_colsum_bf16(DIMS[l + 1], m, p(dt), M, p(gb), sp))
+        assert torch.equal(net.gW[l], gw), l
+        assert torch.equal(net.gb[l], gb), l
+        if l:
+            dn, dnt = z16(M, 256), z16(256, M)
+            gemm(lib, sp, d, net.Wt[l], M, 256, k, gelu_grad_of=net.Z[l - 1], out_bf16=dn, out_bf16_t=dnt)
+            assert torch.equal(net.dZt[l - 1], dnt), l
+            d, dt, k = dn, dnt, 256
+    torch.cuda.synchronize()
+    assert int(net.status.item()) == 0
