@@ -586,6 +586,52 @@ int xpbd_iterate_persistent(const XpbdParams* prm, const XpbdTiles* tiles, const
  * can be resident at once (the largest tile range one launch can take). */
 int xpbd_persistent_fits(const XpbdParams* prm, const XpbdTiles* tiles, int32_t* fits, int32_t* slots);
 
+/* The exchange of partial sums between tiles in xpbd_frame_persistent.  A copy
+ * is a tile's entry of a vertex in tile_verts (n_copies = tile_vptr[n_tiles]).
+ * items[item_ptr[t] ..]: for every copy c of tile t whose vertex other tiles
+ * hold too, one pair (a copy in another tile, c - tile_vptr[t]) per such tile.
+ * slots: two 16-byte mailboxes per copy; tile_cnt: iterations each tile has
+ * run.  Both all zero before the first call, and zeroed together after a
+ * timeout.  A vertex may collect at most 65,535 active constraints per tile. */
+typedef struct XpbdExchange {
+    const int32_t* item_ptr; /* [n_tiles+1] */
+    const int32_t* items;    /* [item_ptr[n_tiles]][2] */
+    int32_t* slots;          /* [2][n_copies][4] */
+    uint32_t* tile_cnt;      /* [n_tiles] */
+    int64_t n_copies;
+    int32_t max_items;       /* most items of a tile */
+    int32_t reserved;
+} XpbdExchange;
+
+/* A frame's substeps: before the iterations of substep 0 first_ops, of every
+ * later one sub_ops, after the last one last_ops (XPBD_OP_* as in
+ * xpbd_vertex_step; all zero: iterations only, pprev and vel untouched);
+ * n_iters Jacobi iterations each.  XPBD_OP_SDF reads *sdf or, for a batch,
+ * each vertex's own grid of *sdf_batch (exactly one set). */
+typedef struct XpbdFrame {
+    int32_t n_sub, n_iters;
+    uint32_t first_ops, sub_ops, last_ops;
+    int32_t reserved;
+    const XpbdSdf* sdf;
+    const XpbdSdfBatch* sdf_batch;
+    const XpbdExchange* ex;
+} XpbdFrame;
+
+/* n_sub x (xpbd_vertex_step + n_iters fused Jacobi iterations as in
+ * xpbd_iterate_persistent) + xpbd_vertex_step in one cooperative launch per
+ * tile range (MultiGridSim.step_frame, mg.py:1409-1418, without multigrid,
+ * fascia or per-iteration hooks; MuscleSim.step, musclesim.py:107-142).  pos,
+ * pprev and vel are written once, at the end.  Of ps it needs tile_own, status
+ * and the tile range; with ring and sync set, launches may alternate with
+ * xpbd_iterate_persistent's on the same words.  A tile waits for its neighbours' sums at most about a
+ * second; then XPBD_STATUS_BARRIER_TIMEOUT is set and the kernel runs to its
+ * end without waiting.  tile_variant's prefetch and packed bits are ignored. */
+int xpbd_frame_persistent(const XpbdParams* prm, const XpbdTiles* tiles, const XpbdVerts* v, const XpbdPersist* ps,
+                          const XpbdFrame* f, xpbd_stream_t stream);
+/* As xpbd_persistent_fits, for xpbd_frame_persistent. */
+int xpbd_frame_fits(const XpbdParams* prm, const XpbdTiles* tiles, const XpbdExchange* ex, int32_t* fits,
+                    int32_t* slots);
+
 /* ---- Learned coarse correction: the per-cage-vertex MLP's kernels.  These
  * have no counterpart in the reference (its solver has no learned part); they
  * serve the learned warm start of the cage (forward, backward, Adam). ---- */

@@ -107,6 +107,17 @@ class XpbdSdfBatch(C.Structure):
                 ("max_push", C.c_float)]
 
 
+class XpbdExchange(C.Structure):
+    _fields_ = [("item_ptr", C.c_void_p), ("items", C.c_void_p), ("slots", C.c_void_p), ("tile_cnt", C.c_void_p),
+                ("n_copies", C.c_int64), ("max_items", C.c_int32), ("reserved", C.c_int32)]
+
+
+class XpbdFrame(C.Structure):
+    _fields_ = [("n_sub", C.c_int32), ("n_iters", C.c_int32), ("first_ops", C.c_uint32), ("sub_ops", C.c_uint32),
+                ("last_ops", C.c_uint32), ("reserved", C.c_int32), ("sdf", C.c_void_p), ("sdf_batch", C.c_void_p),
+                ("ex", C.c_void_p)]
+
+
 class XpbdGemm(C.Structure):
     _fields_ = [("a", C.c_void_p), ("b", C.c_void_p), ("lda", C.c_int32), ("ldb", C.c_int32), ("m", C.c_int32),
                 ("n", C.c_int32), ("k", C.c_int32), ("act", C.c_int32), ("bias", C.c_void_p),
@@ -184,6 +195,10 @@ _SIGS = {
                                  C.POINTER(XpbdPersist), C.c_int32, P], C.c_int),
     "xpbd_persistent_fits": ([C.POINTER(XpbdParams), C.POINTER(XpbdTiles), C.POINTER(C.c_int32),
                               C.POINTER(C.c_int32)], C.c_int),
+    "xpbd_frame_persistent": ([C.POINTER(XpbdParams), C.POINTER(XpbdTiles), C.POINTER(XpbdVerts),
+                               C.POINTER(XpbdPersist), C.POINTER(XpbdFrame), P], C.c_int),
+    "xpbd_frame_fits": ([C.POINTER(XpbdParams), C.POINTER(XpbdTiles), C.POINTER(XpbdExchange), C.POINTER(C.c_int32),
+                         C.POINTER(C.c_int32)], C.c_int),
     "xpbd_gemm_bf16": ([C.POINTER(XpbdGemm), C.c_int32, P], C.c_int),
     "xpbd_colsum_bf16": ([C.c_int32, C.c_int32, P, C.c_int32, P, P], C.c_int),
     "xpbd_adam": ([C.c_int32, C.c_int32, P, P, C.c_int32, P, P, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32,

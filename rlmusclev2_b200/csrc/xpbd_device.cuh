@@ -293,39 +293,52 @@ __device__ __forceinline__ bool con_arapsvd(const float4 p[4], const M3& B, cons
     g[3] = (-g[0] - g[1]) - g[2];
     const float wraw = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
     if (wraw == 0.f) return false;
-    const float dL = -C / (wraw * (invC * invC) + at);
+    const float dL = __fdividef(-C, wraw * (invC * invC) + at);
     const float k = dL * invC * scale;
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = acc[i] + (k * p[i].w) * g[i];
     return true;
 }
 
-// solve_tetvolume_kernel + tet_volume_update_xpbd_fn, solve_kernels.py:553-585, 187-281.
-__device__ __forceinline__ bool con_volume(const float4 p[4], const float4* q, float V0, float k, float kd, float dt,
-                                           float scale, float3 (&acc)[4]) {
-    const float3 p3 = f3(p[3]);
-    const float3 d0 = f3(p[0]) - p3, d1 = f3(p[1]) - p3, d2 = f3(p[2]) - p3;
-    float3 g[4];
-    g[0] = cross(d1, d2) / 6.f;
-    g[1] = cross(d2, d0) / 6.f;
-    g[2] = cross(d0, d1) / 6.f;
-    g[3] = -((g[0] + g[1]) + g[2]);
-    const float ws = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
-    if (!(ws > 1e-9f)) return false;
-    const float volume = dot(cross(d0, d1), d2) / 6.f;
+// What a constraint's stiffness, damping ratio and dt fix: alpha~ = (1 / k) /
+// dt^2 and the damping factor alpha~ beta / dt (0 undamped), beta = k kd dt^2,
+// in the reference's operation order.  Dependent divisions, so the kernels
+// keep them per material instead of forming them per tet or vertex.
+__device__ __forceinline__ float2 xpbd_consts(float k, float kd, float dt) {
     float alpha = 1.f / k;
     alpha = alpha / (dt * dt);
-    const float C = volume - V0;
-    float dsum = 0.f, gamma = 1.f;
+    float gamma = 0.f;
     if (kd > 0.f) {
         const float beta = k * kd * dt * dt;
         gamma = alpha * beta / dt;
+    }
+    return make_float2(alpha, gamma);
+}
+
+// solve_tetvolume_kernel + tet_volume_update_xpbd_fn, solve_kernels.py:553-585,
+// 187-281; c = xpbd_consts of the material.
+__device__ __forceinline__ bool con_volume(const float4 p[4], const float4* q, float V0, float2 c, bool damped,
+                                           float scale, float3 (&acc)[4]) {
+    const float3 p3 = f3(p[3]);
+    const float3 d0 = f3(p[0]) - p3, d1 = f3(p[1]) - p3, d2 = f3(p[2]) - p3;
+    constexpr float kSixth = 1.f / 6.f;
+    float3 g[4];
+    g[0] = kSixth * cross(d1, d2);
+    g[1] = kSixth * cross(d2, d0);
+    g[2] = kSixth * cross(d0, d1);
+    g[3] = -((g[0] + g[1]) + g[2]);
+    const float ws = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
+    if (!(ws > 1e-9f)) return false;
+    const float volume = dot(g[2], d2);
+    const float C = volume - V0;
+    float dsum = 0.f, gamma = 1.f;
+    if (damped) {
         dsum = dot(g[0], f3(p[0]) - f3(q[0])) + dot(g[1], f3(p[1]) - f3(q[1])) + dot(g[2], f3(p[2]) - f3(q[2])) +
                dot(g[3], f3(p[3]) - f3(q[3]));
-        dsum = dsum * gamma;
-        gamma = gamma + 1.f;
+        dsum = dsum * c.y;
+        gamma = c.y + 1.f;
     }
-    const float dl = (-C - dsum) / (gamma * ws + alpha) * scale;
+    const float dl = __fdividef(-C - dsum, gamma * ws + c.x) * scale;
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = acc[i] + (dl * p[i].w) * g[i];
     return true;
@@ -334,9 +347,9 @@ __device__ __forceinline__ bool con_volume(const float4 p[4], const float4* q, f
 // solve_tet_aniso_arap_kernel, solve_kernels.py:1310-1426.  f0 is the
 // normalised mean fiber direction of the tet's 4 vertices (static, built at
 // upload); a zero f0 marks a tet whose mean fiber vanished (fn < 1e-9).
+// at = (1 / (k kscale)) / dt^2 of the material.
 __device__ __forceinline__ bool con_aniso(const float4 p[4], const M3& B, const M3& F, float3 f0, float tendon,
-                                          float act, float k, float ratio, float kscale, float dt, float scale,
-                                          float3 (&acc)[4]) {
+                                          float act, float at, float ratio, float scale, float3 (&acc)[4]) {
     const float3 d = make_float3(F.m[0][0] * f0.x + F.m[0][1] * f0.y + F.m[0][2] * f0.z,
                                  F.m[1][0] * f0.x + F.m[1][1] * f0.y + F.m[1][2] * f0.z,
                                  F.m[2][0] * f0.x + F.m[2][1] * f0.y + F.m[2][2] * f0.z);
@@ -348,7 +361,7 @@ __device__ __forceinline__ bool con_aniso(const float4 p[4], const M3& B, const 
     const float fiberscale = 1.f - belly * act * ratio;
     const float diff = s - fiberscale;
     const float C = 0.5f * diff * diff;
-    const float gs = diff / s;
+    const float gs = __fdividef(diff, s);
     const float dd[3] = {d.x, d.y, d.z}, ff[3] = {f0.x, f0.y, f0.z};
     M3 G;
 #pragma unroll
@@ -362,9 +375,7 @@ __device__ __forceinline__ bool con_aniso(const float4 p[4], const M3& B, const 
     g[3] = (-g[0] - g[1]) - g[2];
     const float wsum = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
     if (wsum < 1.0e-20f) return false;
-    const float sv = k * kscale;
-    const float at = (1.f / sv) / (dt * dt);
-    const float dL = -C / (wsum + at) * scale;
+    const float dL = __fdividef(-C, wsum + at) * scale;
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = acc[i] + (dL * p[i].w) * g[i];
     return true;
@@ -446,27 +457,25 @@ __device__ __forceinline__ bool con_snh(const float4 p[4], const float4* q, cons
 }
 
 // attach_bilateral_update_fn (Jacobi branch), solve_kernels.py:462-526, for
-// restlength-parameterised point attachment to a target.  Returns the delta
-// for the attached vertex.
-__device__ __forceinline__ bool con_attach(float4 p, float3 prev, float3 tgt, float restlength, float k, float kd,
-                                           float dt, float3& out) {
+// restlength-parameterised point attachment to a target; c = xpbd_consts of
+// its material.
+// Returns the delta for the attached vertex.
+__device__ __forceinline__ bool con_attach(float4 p, float3 prev, float3 tgt, float restlength, float2 c, bool damped,
+                                           float3& out) {
     const float im = p.w;
     if (im == 0.f) return false;
     float3 n = f3(p) - tgt;
     const float d = len(n);
     if (!(d >= 1.0e-6f)) return false;
-    float alpha = 1.f / k;
-    alpha = alpha / (dt * dt);
+    const float alpha = c.x;
     const float C = d - restlength;
-    n = n / d;
+    n = __fdividef(1.f, d) * n;
     float dsum = 0.f, gamma = 1.f;
-    if (kd > 0.f) {
-        const float beta = k * kd * dt * dt;
-        gamma = alpha * beta / dt;
-        dsum = gamma * dot(n, f3(p) - prev);
-        gamma = gamma + 1.f;
+    if (damped) {
+        dsum = c.y * dot(n, f3(p) - prev);
+        gamma = c.y + 1.f;
     }
-    const float dL = (-C - dsum) / (gamma * im + alpha);
+    const float dL = __fdividef(-C - dsum, gamma * im + alpha);
     const float3 dp = (-dL) * n;
     out = (-im) * dp;
     return true;

@@ -13,7 +13,7 @@ constexpr unsigned kSpinCheck = 64u;       // polls between two reads of the sta
 // Barrier words (four uint32, zero before the first launch that uses them):
 //   [0], [1]  arrival counters; consecutive launches alternate between them
 //   [2]       free for the kernel (the persistent pass keeps its ring phase there)
-//   [3]       which counter the next launch uses (bit 0)
+//   [3]       which counter the next launch uses (bit 0; the other bits are the kernel's)
 // A launch reads [3] once per CTA before its first arrival, counts every
 // arrival into its counter and waits until the counter reaches k * gridDim.x
 // at its k-th barrier; the counter only grows within a launch, so the last

@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(kThreads, MINB)
         bar = grid_barrier_begin(P.sync);
     }
     const uint32_t ops = XPBD_APPLY_ATTACH | XPBD_APPLY_DIVIDE | XPBD_APPLY_PIN;
-    __shared__ float s_arap_at[XPBD_MAX_MATERIALS];
+    __shared__ MatConsts s_mat[XPBD_MAX_MATERIALS];
     __shared__ int s_defer[2 + kDeferCap];
     if (threadIdx.x == 0) s_defer[0] = s_defer[1] = 0;
-    fill_arap_at(prm, s_arap_at);
+    fill_materials(prm, s_mat);
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i = threadIdx.x; i < nvt; i += blockDim.x) {
         const int g = T.tile_verts[vbeg + i];
@@ -145,9 +145,9 @@ __global__ void __launch_bounds__(kThreads, MINB)
         float4* rn = ring + nxt * nv;
         __syncthreads();  // staged or finished positions, zeroed accumulators
         if constexpr (X2 && CSET != CSET_FULL && !DAMP)
-            project_tile_tets_x2<CSET == CSET_VOL>(prm, T, tile, s_pos, s_ax, s_ay, s_az, s_cnt, s_arap_at);
+            project_tile_tets_x2<CSET == CSET_VOL>(prm, T, tile, s_pos, s_ax, s_ay, s_az, s_cnt, s_mat);
         else
-            project_tile_tets<DAMP, CSET, PF>(prm, T, tile, s_pos, s_prev, s_ax, s_ay, s_az, s_cnt, s_arap_at,
+            project_tile_tets<DAMP, CSET, PF>(prm, T, tile, s_pos, s_prev, s_ax, s_ay, s_az, s_cnt, s_mat,
                                               s_defer, it & 1);
         __syncthreads();
         // boundary partial sums first, so their L2 atomics overlap the interior finish
@@ -177,6 +177,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) P.sync[2] = (phase0 + uint32_t(n_iters)) % 3u;
     if (!nsync) grid_barrier_end(P.sync, bar);
+    // bit 1 of the last word: the ring has been written (see xpbd_frame.cu)
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.sync[3] |= 2u;
 }
 
 uint32_t material_union(const XpbdParams* p) {

@@ -11,15 +11,17 @@ namespace xpbd {
 // ---------------------------------------------------------------------------
 // Per-vertex finish of a Jacobi iteration: ATTACH, divide, pin, from the
 // vertex's flags f, attach target at (xyz, restlength), previous position
-// (read only for damped attach) and pin target pin (w != 0: active).
+// (read only for damped attach) and pin target pin (w != 0: active).  att:
+// xpbd_consts of every attach material (fill_attach), or null.
 __device__ __forceinline__ void finish_core(const XpbdParams& prm, int f, float4 at, float4 prevp, float4 pin, float4& p,
-                                            float4 a, uint32_t ops) {
+                                            float4 a, uint32_t ops, const float2* att = nullptr) {
     if ((ops & XPBD_APPLY_ATTACH) && (f & XPBD_VF_ATTACH_MASK) && (f & XPBD_VF_ATTACH_MASK) <= prm.n_attach_materials) {
         const XpbdAttachMaterial& M = prm.attach[(f & XPBD_VF_ATTACH_MASK) - 1];
         if (M.k > 0.f) {
             const float3 prev = M.damp > 0.f ? f3(prevp) : make_float3(0.f, 0.f, 0.f);
             float3 d;
-            if (con_attach(p, prev, f3(at), at.w, M.k, M.damp, prm.dt, d)) {
+            const float2 c = att ? att[(f & XPBD_VF_ATTACH_MASK) - 1] : xpbd_consts(M.k, M.damp, prm.dt);
+            if (con_attach(p, prev, f3(at), at.w, c, M.damp > 0.f, d)) {
                 a.x += d.x;
                 a.y += d.y;
                 a.z += d.z;
@@ -28,7 +30,7 @@ __device__ __forceinline__ void finish_core(const XpbdParams& prm, int f, float4
         }
     }
     if ((ops & XPBD_APPLY_DIVIDE) && a.w > 1e-9f) {
-        float3 d = make_float3(a.x / a.w, a.y / a.w, a.z / a.w);
+        float3 d = __fdividef(1.f, a.w) * f3(a);
         if (prm.omega != 1.f) d = prm.omega * d;
         p.x += d.x;
         p.y += d.y;
@@ -56,11 +58,26 @@ __device__ __forceinline__ void finish_vertex(const XpbdParams& prm, const XpbdV
 }
 
 // ---------------------------------------------------------------------------
-// Per-material ARAP alpha tilde into shared memory (followed by the caller's
-// __syncthreads before the first projection).
-__device__ __forceinline__ void fill_arap_at(const XpbdParams& prm, float* s_at) {
-    for (int i = threadIdx.x; i < prm.n_materials && i < XPBD_MAX_MATERIALS; i += blockDim.x)
-        s_at[i] = arap_alpha_tilde(prm.materials[i].arap_k, prm.dt);
+// Per-material constants into shared memory (followed by the caller's
+// __syncthreads before the first projection): alpha~ of ARAP and of the fibre
+// term, alpha~ and damping factor of the volume.
+struct MatConsts {
+    float arap, aniso;
+    float2 vol;
+};
+__device__ __forceinline__ void fill_materials(const XpbdParams& prm, MatConsts* s_mat) {
+    for (int i = threadIdx.x; i < prm.n_materials && i < XPBD_MAX_MATERIALS; i += blockDim.x) {
+        const XpbdMaterial& m = prm.materials[i];
+        s_mat[i].arap = arap_alpha_tilde(m.arap_k, prm.dt);
+        s_mat[i].aniso = xpbd_consts(m.aniso_k * prm.fiber_stiffness_scale, 0.f, prm.dt).x;
+        s_mat[i].vol = xpbd_consts(m.vol_k, m.vol_damp, prm.dt);
+    }
+}
+
+// The same for the attach materials' constants.
+__device__ __forceinline__ void fill_attach(const XpbdParams& prm, float2* s_att) {
+    for (int i = threadIdx.x; i < prm.n_attach_materials && i < XPBD_MAX_ATTACH_MATERIALS; i += blockDim.x)
+        s_att[i] = xpbd_consts(prm.attach[i].k, prm.attach[i].damp, prm.dt);
 }
 
 // ---------------------------------------------------------------------------
@@ -100,7 +117,7 @@ constexpr int kDeferCap = 128;
 template <bool DAMP, int CSET, bool PREFETCH = false>
 __device__ __forceinline__ void project_tile_tets(const XpbdParams& prm, const XpbdTiles& T, int tile,
                                                   const float4* s_pos, const float4* s_prev, int* s_ax, int* s_ay,
-                                                  int* s_az, int* s_cnt, const float* s_arap_at,
+                                                  int* s_az, int* s_cnt, const MatConsts* s_mat,
                                                   int* s_defer = nullptr, int parity = 0) {
     const float acc_scale = prm.acc_scale;
     const float arap_skip = arap_skip_threshold(prm.arap_skip_ssq);
@@ -114,7 +131,8 @@ __device__ __forceinline__ void project_tile_tets(const XpbdParams& prm, const X
     // One tet from its streams; `late` = the deferred pass.
     auto project_one = [&](int t, const uint4& q, const float4& b0, const float4& b1, float b2, bool late) {
         const int l[4] = {int(q.x & 0xffffu), int(q.x >> 16), int(q.y & 0xffffu), int(q.y >> 16)};
-        const XpbdMaterial& m = prm.materials[min(int(q.z & 0xffu), XPBD_MAX_MATERIALS - 1)];
+        const int mat = min(int(q.z & 0xffu), XPBD_MAX_MATERIALS - 1);
+        const XpbdMaterial& m = prm.materials[mat];
         const float V0 = __uint_as_float(q.w);
         M3 B;
         B.m[0][0] = b0.x; B.m[0][1] = b0.y; B.m[0][2] = b0.z;
@@ -149,16 +167,14 @@ __device__ __forceinline__ void project_tile_tets(const XpbdParams& prm, const X
             con_snh(p, pq, B, F, V0, m.snh_mu, m.snh_lam, m.snh_damp, prm.dt, acc_scale, d))
             nact += 1;
         if (CSET >= CSET_VOL && (fl & XPBD_MAT_VOLUME) &&
-            con_volume(p, pq, V0, m.vol_k, m.vol_damp, prm.dt, acc_scale, d))
+            con_volume(p, pq, V0, s_mat[mat].vol, DAMP && m.vol_damp > 0.f, acc_scale, d))
             nact += 1;
         if (fl & XPBD_MAT_ANISO) {
             const float4 fb = reinterpret_cast<const float4*>(T.tet_fiber)[t];
-            if (con_aniso(p, B, F, f3(fb), fb.w, T.tet_act[t], m.aniso_k, prm.contraction_ratio,
-                          prm.fiber_stiffness_scale, prm.dt, acc_scale, d))
+            if (con_aniso(p, B, F, f3(fb), fb.w, T.tet_act[t], s_mat[mat].aniso, prm.contraction_ratio, acc_scale, d))
                 nact += 1;
         }
-        if ((fl & XPBD_MAT_ARAPSVD) && con_arapsvd(p, B, F, s_arap_at[min(int(q.z & 0xffu), XPBD_MAX_MATERIALS - 1)],
-                                                   arap_skip, acc_scale, d, all_svd || late))
+        if ((fl & XPBD_MAT_ARAPSVD) && con_arapsvd(p, B, F, s_mat[mat].arap, arap_skip, acc_scale, d, all_svd || late))
             nact += 1;
         if (nact != 0) {
             // Range check on the sum of the 12 scaled |components| (not their

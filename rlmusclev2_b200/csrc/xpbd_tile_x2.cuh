@@ -151,7 +151,7 @@ __device__ __forceinline__ void acc_tet(const int (&l)[4], const float3 (&d)[4],
 template <bool VOL>
 __device__ __forceinline__ void project_tile_tets_x2(const XpbdParams& prm, const XpbdTiles& T, int tile,
                                                      const float4* s_pos, int* s_ax, int* s_ay, int* s_az,
-                                                     int* s_cnt, const float* s_arap_at) {
+                                                     int* s_cnt, const MatConsts* s_mat) {
     const float acc_scale = prm.acc_scale;
     const float arap_skip = arap_skip_threshold(prm.arap_skip_ssq);
     const bool force_svd = (prm.tile_variant & 2) != 0;
@@ -260,7 +260,7 @@ __device__ __forceinline__ void project_tile_tets_x2(const XpbdParams& prm, cons
                 wsum = fma2(w3, vdot2(q3, q3), wsum);
                 acta = acta && wsum.x != 0.f;
                 actb = actb && wsum.y != 0.f;
-                const f2 den = add2(wsum, pk(s_arap_at[ma], s_arap_at[mb]));
+                const f2 den = add2(wsum, pk(s_mat[ma].arap, s_mat[mb].arap));
                 const f2 dL = pk(-__fdividef(C.x, den.x), -__fdividef(C.y, den.y));
                 const f2 s0 = mul2(dL, w0), s1 = mul2(dL, w1), s2 = mul2(dL, w2), s3 = mul2(dL, w3);
                 const V2 e0 = {mul2(s0, q0.x), mul2(s0, q0.y), mul2(s0, q0.z)};
@@ -340,8 +340,7 @@ __device__ __forceinline__ void project_tile_tets_x2(const XpbdParams& prm, cons
             B.m[1][0] = lane ? B10.y : B10.x; B.m[1][1] = lane ? B11.y : B11.x; B.m[1][2] = lane ? B12.y : B12.x;
             B.m[2][0] = lane ? B20.y : B20.x; B.m[2][1] = lane ? B21.y : B21.x; B.m[2][2] = lane ? B22.y : B22.x;
             const float4 fbv = reinterpret_cast<const float4*>(T.tet_fiber)[t];
-            if (con_aniso(pp, B, F, f3(fbv), fbv.w, T.tet_act[t], prm.materials[m].aniso_k, prm.contraction_ratio,
-                          prm.fiber_stiffness_scale, prm.dt, 1.f, dd))
+            if (con_aniso(pp, B, F, f3(fbv), fbv.w, T.tet_act[t], s_mat[m].aniso, prm.contraction_ratio, 1.f, dd))
                 n += 1;
         };
         if (fa & XPBD_MAT_ANISO) aniso(pa, ta, ma, 0, da, na);

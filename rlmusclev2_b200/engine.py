@@ -49,6 +49,28 @@ def max_rest_edge(pos: np.ndarray, tets: np.ndarray) -> float:
     return m
 
 
+def exchange_items(tile_vptr: np.ndarray, tile_verts: np.ndarray, n_verts: int) -> tuple[np.ndarray, np.ndarray]:
+    """The sums every tile fetches from others: (ptr [n_tiles + 1], items
+    [n, 2]), item = (entry of tile_verts in another tile, local vertex of this
+    one), for every ordered pair of tiles that hold the same vertex."""
+    tv = np.asarray(tile_verts, np.int64)
+    nc, nt = tv.shape[0], len(tile_vptr) - 1
+    order = np.argsort(tv, kind="stable")  # entries by vertex, tiles ascending
+    cnt = np.bincount(tv, minlength=n_verts)
+    start = np.concatenate([[0], np.cumsum(cnt)])
+    n_of = cnt[tv]
+    own = np.repeat(np.arange(nc), n_of)  # every entry with every entry of its vertex ...
+    j = np.arange(own.size) - np.repeat(np.cumsum(n_of) - n_of, n_of)
+    other = order[start[tv[own]] + j]
+    keep = other != own  # ... but itself
+    own, other = own[keep], other[keep]
+    tile = np.repeat(np.arange(nt), np.diff(tile_vptr))
+    ptr = np.zeros(nt + 1, np.int32)
+    ptr[1:] = np.cumsum(np.bincount(tile[own], minlength=nt))
+    items = np.stack([other, own - np.asarray(tile_vptr, np.int64)[tile[own]]], 1).astype(np.int32)
+    return ptr, (items if items.size else np.zeros((1, 2), np.int32))
+
+
 def status_error(tile_status: int, dcd_status: int = 0) -> str | None:
     """The error a frame must raise for its status words, or None.
 
@@ -138,6 +160,7 @@ class XpbdEngine:
         self._status_host = torch.zeros(2, dtype=torch.int32).pin_memory()
         self._status_event = None
         self._t_own = T(L.tile_own)
+        self._build_exchange()
         self.use_persistent = True
         self._metrics_buf = torch.zeros(8, dtype=torch.float64, device=dev)  # >= sizeof(XpbdMetrics)
         # tiles
@@ -277,15 +300,45 @@ class XpbdEngine:
         fits, slots = C.c_int32(0), C.c_int32(0)
         capi.check(self._lib.xpbd_persistent_fits(C.byref(self._prm), C.byref(t), C.byref(fits), C.byref(slots)))
         self._persist_slots = int(slots.value)
+        if self._exchange is not None:  # one set of tile ranges for both kinds of launch
+            fslots = C.c_int32(0)
+            capi.check(self._lib.xpbd_frame_fits(C.byref(self._prm), C.byref(t), C.byref(self._exchange),
+                                                 C.byref(fits), C.byref(fslots)))
+            if fslots.value < min(L.n_tiles, self._persist_slots) and not self._persist_ranges(fslots.value):
+                self._exchange = None  # tiles too large for its shared memory
+            else:
+                self._persist_slots = min(self._persist_slots, int(fslots.value))
         self._build_persist(self._persist_slots)
         for g in self._graphs.values():
             capi.check(self._lib.xpbd_graph_destroy(g))
         self._graphs = {}
 
-    #: synchronisation between the iterations of the persistent pass: "grid"
-    #: (one grid-wide barrier) or "neighbour" (each tile waits for the tiles it
-    #: shares boundary vertices with)
-    persistent_sync = "grid"
+    #: how the tiles of a persistent launch pass on their partial sums:
+    #: "exchange" (mailboxes between the tiles that share a vertex; whole frames
+    #: in one launch), or the global accumulator with a grid-wide barrier per
+    #: iteration ("grid") or with each tile waiting for the tiles it shares
+    #: vertices with ("neighbour")
+    persistent_sync = "exchange"
+
+    def _build_exchange(self) -> None:
+        """Mailboxes of the shared vertices (XpbdExchange): per tile the pairs
+        (other tile's entry of a vertex, own local vertex).  None where a vertex
+        could collect more constraints than a slot's 16-bit count holds."""
+        L = self.layout
+        nc = L.tile_verts.shape[0]
+        self._exchange = None
+        if np.bincount(L.tets_new.reshape(-1), minlength=1).max() * 4 > 65535:
+            return
+        ptr, items = exchange_items(L.tile_vptr, L.tile_verts, L.n_verts)
+        dev = self.device
+        self._ex_ptr, self._ex_items = torch.from_numpy(ptr).to(dev), torch.from_numpy(items).to(dev)
+        self._ex_slots = torch.zeros((2, nc, 4), dtype=torch.int32, device=dev)
+        self._ex_cnt = torch.zeros(L.n_tiles, dtype=torch.int32, device=dev)
+        x = capi.XpbdExchange()
+        x.item_ptr, x.items = _ptr(self._ex_ptr), _ptr(self._ex_items)
+        x.slots, x.tile_cnt, x.n_copies = _ptr(self._ex_slots), _ptr(self._ex_cnt), nc
+        x.max_items = int(np.diff(ptr).max())
+        self._exchange = x
 
     def _tile_neighbours(self):
         """CSR of the tiles each tile shares a boundary vertex with (itself excluded)."""
@@ -310,17 +363,17 @@ class XpbdEngine:
         ranges = self._persist_ranges(int(slots))
         if 4 * len(ranges) > self._psync.numel():
             self._psync = torch.zeros(4 * len(ranges), dtype=torch.int32, device=self.device)
-        ptr, idx = self._tile_neighbours()
-        self._t_nbr_ptr = torch.from_numpy(ptr).to(self.device)
-        self._t_nbr_idx = torch.from_numpy(idx if idx.size else np.zeros(1, np.int32)).to(self.device)
+        nb = self.persistent_sync == "neighbour"
+        if nb:
+            ptr, idx = self._tile_neighbours()
+            self._t_nbr_ptr = torch.from_numpy(ptr).to(self.device)
+            self._t_nbr_idx = torch.from_numpy(idx if idx.size else np.zeros(1, np.int32)).to(self.device)
         self._t_cnt = torch.zeros(self.layout.n_tiles, dtype=torch.int32, device=self.device)
         # a vertex's ring slots follow its range's phase word: start all over
         with torch.cuda.stream(self._stream):
-            self._ring.zero_()
-            self._psync.zero_()
+            self._reset_persist()
         self._stream.synchronize()
         self._persist = []
-        nb = self.persistent_sync == "neighbour"
         for k, (b, e) in enumerate(ranges):
             ps = capi.XpbdPersist()
             ps.tile_own, ps.ring, ps.status = _ptr(self._t_own), _ptr(self._ring), _ptr(self._pstatus)
@@ -331,6 +384,15 @@ class XpbdEngine:
                                                        _ptr(self._t_cnt))
             self._persist.append(ps)
         self._persist_fits = bool(ranges)
+
+    def _reset_persist(self) -> None:
+        """Zero the persistent launches' words on the current stream: ring,
+        barriers, tile counters and mailboxes."""
+        for t in (self._ring, self._psync, self._t_cnt):
+            t.zero_()
+        if self._exchange is not None:
+            self._ex_slots.zero_()
+            self._ex_cnt.zero_()
 
     # -------------------------------------------------------------- launches
     def _vstep(self, ops: int) -> None:
@@ -395,6 +457,8 @@ class XpbdEngine:
         when the tiles fit on the GPU at once, else n x _fused_iteration()."""
         if n <= 0:
             return
+        if self._fused_substeps(1, n, 0, 0, 0):
+            return
         if self.use_persistent and self._persist_fits and self.fused_mode == capi.PROJECT_FUSED:
             for ps in self._persist:
                 capi.check(self._lib.xpbd_iterate_persistent(C.byref(self._prm), C.byref(self._tiles),
@@ -402,6 +466,33 @@ class XpbdEngine:
             return
         for _ in range(n):
             self._fused_iteration()
+
+    def _fused_substeps(self, n_sub: int, n_iters: int, first_ops: int, sub_ops: int, last_ops: int) -> bool:
+        """n_sub substeps of (vertex step, n_iters fused iterations) and the
+        last vertex step, in one persistent launch per tile range; False (and
+        nothing launched) where the tiles do not fit at once or the tile
+        variant asks for an instance the frame pass does not have."""
+        if not (self.use_persistent and self._persist_fits and self.fused_mode == capi.PROJECT_FUSED
+                and self.persistent_sync == "exchange" and self._exchange is not None
+                and n_iters > 0 and self.n_cons > 0) or (self._prm.tile_variant & ~0x53):
+            return False
+        f = capi.XpbdFrame()
+        f.n_sub, f.n_iters, f.ex = int(n_sub), int(n_iters), C.addressof(self._exchange)
+        sdf = None
+        if (first_ops | sub_ops | last_ops) & capi.OP_SDF:
+            if self._sdf is None:
+                first_ops, sub_ops, last_ops = (o & ~capi.OP_SDF for o in (first_ops, sub_ops, last_ops))
+            else:
+                sdf = self._sdf.struct()
+                if isinstance(sdf, capi.XpbdSdfBatch):
+                    f.sdf_batch = C.addressof(sdf)
+                else:
+                    f.sdf = C.addressof(sdf)
+        f.first_ops, f.sub_ops, f.last_ops = first_ops, sub_ops, last_ops
+        for ps in self._persist:
+            capi.check(self._lib.xpbd_frame_persistent(C.byref(self._prm), C.byref(self._tiles), C.byref(self._verts),
+                                                       C.byref(ps), C.byref(f), self._sp))
+        return True
 
     def persistent_status(self, reset: bool = True) -> int:
         """XPBD_STATUS_* bits of the persistent pass and of the tile passes'
@@ -412,9 +503,7 @@ class XpbdEngine:
         self._status_pending = False  # this read supersedes the copy queued behind the last frame
         if st and reset:
             with torch.cuda.stream(self._stream):
-                self._ring.zero_()
-                self._psync.zero_()
-                self._t_cnt.zero_()
+                self._reset_persist()
                 self._pstatus.zero_()
             self._stream.synchronize()
         return st
@@ -451,9 +540,7 @@ class XpbdEngine:
         if msg is None:
             return
         with torch.cuda.stream(self._stream):
-            self._ring.zero_()
-            self._psync.zero_()
-            self._t_cnt.zero_()
+            self._reset_persist()
             self._pstatus.zero_()
             dcd = getattr(self, "dcd", None)
             if dcd is not None:

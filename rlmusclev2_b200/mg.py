@@ -818,6 +818,10 @@ class MultiGridSim(MuscleSim):
         self.apply_pintotarget_all()
         vel = 0 if self.quasi_static else capi.OP_VELOCITY
         push = capi.OP_SDF if sdf is not None else 0
+        if self.mg is None and self.fascia is None and not self.n_m2m and not self.collision_solvers_iter:
+            if self._fused_substeps(self.nsubsteps, self.fine_iters, capi.OP_PREDICT | pin,
+                                    capi.OP_PREDICT | pin | push | vel, push | vel):
+                return
         for sub in range(self.nsubsteps):
             if self.mg is None:
                 self._vstep(capi.OP_PREDICT | pin | ((push | vel) if sub > 0 else 0))

@@ -367,9 +367,12 @@ class MuscleSim(XpbdEngine):
                 or (float(self._option("repair_alpha", 0.0)) > 0.0 and int(self._option("repair_iters", 0)) > 0))
 
     def _frame_fused(self) -> None:
-        """One frame, fused: [predict] (tile pass + boundary finish) ... with the
-        velocity update of substep s folded into the prediction of s+1."""
+        """One frame, fused: one persistent launch over all substeps where the
+        tiles fit at once, else [predict] (tile pass + boundary finish) ... with
+        the velocity update of substep s folded into the prediction of s+1."""
         n = self.num_substeps
+        if self._fused_substeps(n, 1, capi.OP_PREDICT, capi.OP_PREDICT | capi.OP_VELOCITY, capi.OP_VELOCITY):
+            return
         for sub in range(n):
             ops = capi.OP_PREDICT | (capi.OP_VELOCITY if sub > 0 else 0)
             self._vstep(ops)

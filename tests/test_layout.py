@@ -78,3 +78,21 @@ def test_fiber_f0_normalised():
     vf = np.tile(np.array([[0, 0, 1]], np.float32), (m.verts.shape[0], 1))
     f0 = fiber_f0(vf, m.tets)
     np.testing.assert_allclose(f0, np.tile([0, 0, 1], (m.tets.shape[0], 1)), atol=1e-7)
+
+
+@pytest.mark.parametrize("tile_tets", [64, 300, 100000])
+def test_exchange_items_list_every_other_tile_of_a_vertex(tile_tets):
+    """Every tile fetches, for each vertex it shares, one sum from each other tile that holds it."""
+    from rlmusclev2_b200.engine import exchange_items
+    from rlmusclev2_b200.meshgen import box_muscle
+    m = box_muscle(4, 3, 7)
+    t = collect_raw_constraints(m.verts, m.tets, [dict(type="tetarapsvd", name="arap", stiffness=1e6)]).sorted_by_type()
+    L = build_layout(m.verts, m.tets, t, tile_tets=tile_tets)
+    ptr, items = exchange_items(L.tile_vptr, L.tile_verts, L.n_verts)
+    tile = np.repeat(np.arange(L.n_tiles), np.diff(L.tile_vptr))
+    want = set()
+    for v in range(L.n_verts):
+        c = np.nonzero(L.tile_verts == v)[0]
+        want |= {(int(tile[a]), int(b), int(a - L.tile_vptr[tile[a]])) for a in c for b in c if a != b}
+    got = [(k, int(o), int(i)) for k in range(L.n_tiles) for o, i in items[ptr[k]:ptr[k + 1]]]
+    assert len(got) == len(set(got)) and set(got) == want
