@@ -366,6 +366,7 @@ class MultiGridSim(MuscleSim):
         self._h2d_event = torch.cuda.Event()
         self._h2d_event.record(self._stream)
         self._presub_idx = None  # constraint points of the soft pin: all vertices
+        self._reproject = False  # this frame re-projects the slide binding
         if self._host_tgt:
             self._pts_tgt = torch.zeros((self.NV, 3), dtype=torch.float32, device=dev)
             self._pts_host = torch.zeros((self.NV, 3), dtype=torch.float32).pin_memory()
@@ -795,12 +796,18 @@ class MultiGridSim(MuscleSim):
         self.apply_pintotarget_all()
 
     def _fusable(self) -> bool:
+        """One captured graph serves every frame (a sliding binding needs two:
+        with and without the re-projection)."""
+        return self._program_fusable() and not getattr(self, "use_sliding", False)
+
+    def _program_fusable(self) -> bool:
+        """The frame's program has device launches only."""
         cs = getattr(self, "collision_solvers", None) or []
         its = getattr(self, "collision_solvers_iter", None) or []
         dcd = getattr(self, "dcd", None)
         return (all(dcd is not None and fn == dcd.solve for fn in its) and not getattr(self, "constraint_solvers", None)
                 and all(getattr(c, "graph_safe", False) for c in cs) and len(cs) <= 1
-                and getattr(self, "program", None) is None and not getattr(self, "use_sliding", False))
+                and getattr(self, "program", None) is None)
 
     def _frame_fused(self) -> None:
         self._targets_kernel()
@@ -869,8 +876,9 @@ class MultiGridSim(MuscleSim):
         self._check_status()
         if self._frame_loaded != frame:
             self.load_frame_targets(frame)
-        if self._fusable():
-            self._graph("frame", self._frame_fused)
+        if self._program_fusable():
+            # frames that re-project the slide binding launch another targets kernel
+            self._graph(("frame", self._reproject), self._frame_fused)
         else:
             self._kinematic_step(frame)
             if self.fascia is not None:
