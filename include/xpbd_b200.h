@@ -488,21 +488,21 @@ typedef struct XpbdDcd {
     float* x_prev;            /* [n_verts][4] positions at the broadphase (friction reference) */
     float* dP;                /* [n_verts][4] response accumulator, zero between calls */
     int32_t* status;          /* [1] XPBD_STATUS_* bits */
-    float* ws_nodes;          /* workspace: BVH node records (children's boxes) + leaf boxes */
+    float* ws_nodes;          /* workspace: leaf records (box, id, group, vertices) in Morton order */
     uint32_t* ws_keys;        /* [n_tris] Morton keys (sorted in place) */
     int32_t* ws_vals;         /* [n_tris] triangle ids in Morton order */
-    uint32_t* ws_keys2;       /* [n_tris] sort ping-pong */
+    uint32_t* ws_keys2;       /* [n_tris] sort ping-pong, then pairs per 32 queries and their offsets */
     int32_t* ws_vals2;        /* [n_tris] */
-    int32_t* ws_hist;         /* radix histograms, scan scratch and the sort's four grid barrier words (its last
+    int32_t* ws_hist;         /* radix histograms and the sort's four grid barrier words (its last
                                  four entries); zero before the first call */
     float* ws_bbox;           /* boxes of 32- and 1024-leaf Morton blocks (2 float4 each) */
-    int32_t* ws_count;        /* [n_tris] pairs per Morton position, then their offsets */
+    int32_t* ws_count;        /* [n_tris] pairs per Morton position */
     int32_t* ws_total;        /* [1] */
     int32_t* ws_slots;        /* [16][n_tris] first partners of each query (counting pass) */
-    int32_t* ws_split;        /* [n_tris-1][4] leaf range and split of each internal node */
-    int32_t refit_only;       /* 1: keep the Morton order and hierarchy of the last rebuild on this
-                                 workspace and recompute the boxes only (same pair set; no sort, no
-                                 split search).  Needs one earlier call with 0. */
+    int32_t* ws_split;        /* unused (16-byte aligned, not null) */
+    int32_t refit_only;       /* 1: keep the Morton order of the last rebuild on this workspace and
+                                 recompute the boxes only (same pair set; no sort).  Needs one earlier
+                                 call with 0. */
 } XpbdDcd;
 
 /* Element counts of the DCD workspace arrays for n_tris triangles. */
@@ -512,8 +512,9 @@ typedef struct XpbdDcdWorkspaceSizes {
 
 int xpbd_dcd_workspace_query(int32_t n_tris, XpbdDcdWorkspaceSizes* out);
 
-/* AABBs, LBVH rebuild (Morton sort + Karras hierarchy + refit) and the
- * candidate pair list; snapshot_prev != 0 first copies pos4 to x_prev
+/* AABBs in Morton order with the boxes of 32- and 1024-leaf blocks, and the
+ * candidate pair list (grouped by the pair's first triangle in Morton order,
+ * partners in Morton order); snapshot_prev != 0 first copies pos4 to x_prev
  * (UdcfDcdCollider.solve with i_iter == 0, udcf/solver.py:365-382). */
 int xpbd_dcd_broadphase(const XpbdDcd* dcd, const float* pos4, int32_t snapshot_prev, xpbd_stream_t stream);
 

@@ -142,8 +142,8 @@ class UdcfParams:
     gauss_seidel: bool = False
     max_push: float = 0.0
     use_bvh: bool = True
-    # Library-specific: rebuild the LBVH (Morton sort + hierarchy) every n-th
-    # broadphase and refit the boxes in between.  1 = the reference's
+    # Library-specific: rebuild the Morton order every n-th broadphase and only
+    # recompute the boxes in between.  1 = the reference's
     # per-broadphase rebuild; the pair set is the same for any n.
     bvh_rebuild_every: int = 1
 
@@ -202,22 +202,19 @@ class DcdBuffers:
         self.d = d
 
     def broadphase(self, pos4: torch.Tensor, snapshot_prev: bool, stream, refit_only: bool = False) -> None:
-        """Boxes, LBVH and pair list; ``refit_only`` keeps the last rebuild's
-        Morton order and hierarchy (the first call always rebuilds)."""
+        """Boxes and pair list; ``refit_only`` keeps the last rebuild's Morton
+        order (the first call always rebuilds)."""
         self.d.refit_only = int(bool(refit_only) and self._built)
         capi.check(self.lib.xpbd_dcd_broadphase(C.byref(self.d), C.c_void_p(pos4.data_ptr()), int(snapshot_prev),
                                                 stream))
         self._built = True
 
     def broadphase_launches(self, snapshot_prev: bool = True, refit_only: bool = False) -> int:
-        """Kernels one xpbd_dcd_broadphase call launches: snapshot copy, boxes,
-        cooperative sort (not when refitting), leaf permute, build or refit,
-        counting traversal, the count scan (2 launches, 3 above 4096
-        triangles), fill pass, total."""
-        n = int(self.d.n_tris)
-        scan = 2 + (1 if n > 4096 else 0)
-        sort = 0 if refit_only else 1
-        return int(snapshot_prev) + 2 + sort + (1 if n > 1 else 0) + 1 + scan + 2
+        """Kernels one xpbd_dcd_broadphase call launches: keys and snapshot
+        (neither: no launch), cooperative sort (not when refitting), leaves,
+        counting pass, scan, fill pass."""
+        rebuild = 0 if refit_only else 1
+        return int(bool(snapshot_prev) or bool(rebuild)) + rebuild + 4
 
     def narrow_respond(self, pos4: torch.Tensor, stream) -> None:
         capi.check(self.lib.xpbd_dcd_narrow_respond(C.byref(self.d), C.c_void_p(pos4.data_ptr()), stream))

@@ -1,12 +1,18 @@
 // Triangle-triangle discrete collision detection (DCD) for sm_100a.
 //
-// Broadphase: per-triangle AABBs padded by the thickness, 30-bit Morton codes
-// of their centres, a stable LSD radix sort (8-bit digits, per-warp ranking
-// with __match_any_sync), a linear BVH built with Karras' method ("Maximizing
-// Parallelism in the Construction of BVHs, Octrees, and k-d Trees", HPG 2012)
-// and refitted bottom-up with per-node arrival counters; then a two-pass
-// traversal (count, exclusive scan, fill) that lists the AABB-overlapping
-// pairs (i, j > i) of every triangle in a deterministic order.
+// Broadphase: 24-bit Morton codes of the triangles' padded boxes, a stable LSD
+// radix sort (8-bit digits, per-warp ranking with __match_any_sync), the boxes
+// in Morton order together with those of every 32 and every 1024 consecutive
+// leaves, and a block traversal: a warp takes 32 consecutive triangles and
+// walks down from the 1024-leaf blocks that their boxes touch to 32-leaf blocks,
+// and each triangle meets the 32 leaves of a block at once.  Two passes (count,
+// scan, fill) list the pairs in a deterministic order, by query and partner
+// position.
+//
+// A binary tree (Karras' construction, a query per thread) needed a build
+// launch of 32 us and left 11 of 32 lanes active on chains of dependent node
+// loads: 70 us for the counting pass of 105k triangles, the block traversal
+// takes 51 us, most of it in the warps at jumps of the curve.
 //
 // Narrowphase / response / apply restate the reference's UDCF kernels
 // (collision/udcf/kernel.py:164-474, 713-822): Moller interval rejection,
@@ -26,25 +32,28 @@ using namespace xpbd;
 namespace {
 
 constexpr int kSortThreads = 1024;  // keys per scatter round; the sort's CTA size
-constexpr int kScanItems = 4;     // consecutive elements per thread in the block scan
-constexpr int kScanBlock = 1024 * kScanItems;
-constexpr int kStack = 64;
+constexpr int kScanItems = 4;       // consecutive elements per thread and round of the scan
 constexpr int kSlots = 16;  // partners a query keeps from the counting pass
+constexpr int kNarrowCtas = 592;  // 4 x 148 SMs
 constexpr float kThresh = 1.0e-5f;  // udcf/kernel.py:40 THRESH
-
-struct Aabb {
-    float3 lo, hi;
-};
 
 __device__ __forceinline__ float4 ld4(const float* p, int i) { return reinterpret_cast<const float4*>(p)[i]; }
 
-// ws_nodes layout (float4 units): internal node records [4 (n-1)), then the
-// leaf boxes in Morton order [2 n), then the leaf boxes in triangle order
-// [2 n).  Record i holds its two children: lo_a (w: last Morton position
-// under a), hi_a (w: a's node id), lo_b, hi_b; node ids >= n-1 are leaves
-// (position id - (n-1)).  A visit is one 64-byte load.
-__host__ __device__ __forceinline__ int64_t sorted_leaf_base(int n) { return int64_t(4) * (n - 1); }
-__host__ __device__ __forceinline__ int64_t tri_leaf_base(int n) { return int64_t(4) * (n - 1) + 2 * int64_t(n); }
+// ws_nodes: three float4 arrays of the leaves in Morton order: box lo (w: the
+// triangle id), box hi (w: its group), vertex ids.  ws_bbox: boxes (lo, hi) of
+// the 32-leaf blocks, then of the 1024-leaf blocks.  ws_keys2 (free after the
+// sort): pairs per 32-query block, then their offsets.
+struct Leaves {
+    float4 *lo, *hi;
+    int4* verts;
+    float4 *b32, *b1k;
+    __device__ __forceinline__ explicit Leaves(const XpbdDcd& D)
+        : lo(reinterpret_cast<float4*>(D.ws_nodes)),
+          hi(lo + D.n_tris),
+          verts(reinterpret_cast<int4*>(hi + D.n_tris)),
+          b32(reinterpret_cast<float4*>(D.ws_bbox)),
+          b1k(b32 + 2 * ((D.n_tris + 31) / 32)) {}
+};
 
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
     v &= 0x3ffu;
@@ -55,44 +64,41 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
     return v;
 }
 
-// ---------------------------------------------------------------- AABBs
-// KEYS = false (refit-only broadphase): boxes only; the Morton keys and the
-// sorted order of the last rebuild are kept.
-template <bool KEYS>
-__global__ void k_tri_aabb(XpbdDcd D, const float* __restrict__ pos4) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.n_tris) return;
-    const int a = D.tris[3 * i], b = D.tris[3 * i + 1], c = D.tris[3 * i + 2];
+// ---------------------------------------------------------------- boxes
+// tri_aabb_kernel (udcf/kernel.py:917-934)
+__device__ __forceinline__ void tri_box(const XpbdDcd& D, const float* pos4, int a, int b, int c, float3& lo, float3& hi) {
     const float3 pa = f3(ld4(pos4, a)), pb = f3(ld4(pos4, b)), pc = f3(ld4(pos4, c));
     const float t = D.thickness;
-    // tri_aabb_kernel (udcf/kernel.py:917-934)
-    const float3 lo = make_float3(fminf(fminf(pa.x, pb.x), pc.x) - t, fminf(fminf(pa.y, pb.y), pc.y) - t,
-                                  fminf(fminf(pa.z, pb.z), pc.z) - t);
-    const float3 hi = make_float3(fmaxf(fmaxf(pa.x, pb.x), pc.x) + t, fmaxf(fmaxf(pa.y, pb.y), pc.y) + t,
-                                  fmaxf(fmaxf(pa.z, pb.z), pc.z) + t);
-    float4* tri_box = reinterpret_cast<float4*>(D.ws_nodes) + tri_leaf_base(D.n_tris);
-    tri_box[2 * i] = make_float4(lo.x, lo.y, lo.z, 0.f);
-    tri_box[2 * i + 1] = make_float4(hi.x, hi.y, hi.z, 0.f);
-    if (!KEYS) return;
-    const float3 cen = make_float3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
-    float q[3] = {cen.x, cen.y, cen.z};
+    lo = make_float3(fminf(fminf(pa.x, pb.x), pc.x) - t, fminf(fminf(pa.y, pb.y), pc.y) - t,
+                     fminf(fminf(pa.z, pb.z), pc.z) - t);
+    hi = make_float3(fmaxf(fmaxf(pa.x, pb.x), pc.x) + t, fmaxf(fmaxf(pa.y, pb.y), pc.y) + t,
+                     fmaxf(fmaxf(pa.z, pb.z), pc.z) + t);
+}
+
+// Morton keys into the buffers the first of the sort's three passes reads (8
+// bits per axis: cells of 3.5 mm on the 0.9-m body, about half a triangle; the
+// order only decides how tight the leaf blocks are), and the snapshot of the
+// positions when asked for.
+__global__ void k_tri_keys(XpbdDcd D, const float* __restrict__ pos4, int keys, int snapshot) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (snapshot && i < D.n_verts) reinterpret_cast<float4*>(D.x_prev)[i] = ld4(pos4, i);
+    if (!keys || i >= D.n_tris) return;
+    float3 lo, hi;
+    tri_box(D, pos4, D.tris[3 * i], D.tris[3 * i + 1], D.tris[3 * i + 2], lo, hi);
+    const float q[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
     uint32_t code = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float ext = fmaxf(D.box_hi[k] - D.box_lo[k], 1e-30f);
-        float u = (q[k] - D.box_lo[k]) / ext * 1023.f;
-        u = fminf(fmaxf(u, 0.f), 1023.f);
+        float u = (q[k] - D.box_lo[k]) / ext * 255.f;
+        u = fminf(fmaxf(u, 0.f), 255.f);
         code |= spread10(uint32_t(u)) << k;
     }
-    D.ws_keys[i] = code;
-    D.ws_vals[i] = i;
+    D.ws_keys2[i] = code;
+    D.ws_vals2[i] = i;
 }
 
 // ---------------------------------------------------------- radix sort
-// Exclusive scan in three launches: per-block scans of kScanBlock elements
-// (each thread a run of kScanItems, warp shuffles across threads) leaving
-// block totals in sums[], one CTA scanning sums[], and a launch adding each
-// block's offset.  total (optional) receives the sum of all elements.
 __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int* block_total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int x = v;
@@ -116,61 +122,42 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int* block
     return incl - v;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_blocks(int* __restrict__ a, int n, int* __restrict__ sums) {
+// One CTA: the pair counts of the query blocks become offsets (a 32nd of the
+// triangles: 3,287 values at 105k), their sum the pair count.
+__global__ void __launch_bounds__(1024) k_scan_pairs(XpbdDcd D) {
     __shared__ int warp_sums[32];
-    __shared__ int total;
-    const int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
-    int v[kScanItems];
-    int run = 0;
-#pragma unroll
-    for (int q = 0; q < kScanItems; ++q) {
-        v[q] = base + q < n ? a[base + q] : 0;
-        run += v[q];
-    }
-    int off = block_excl_scan(run, warp_sums, &total);
-#pragma unroll
-    for (int q = 0; q < kScanItems; ++q) {
-        if (base + q < n) a[base + q] = off;
-        off += v[q];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(1024) k_scan_sums(int* __restrict__ sums, int nb, int* __restrict__ total) {
-    __shared__ int warp_sums[32];
-    __shared__ int carry;
+    __shared__ int carry, round_total;
+    int* a = reinterpret_cast<int*>(D.ws_keys2);
+    const int nb = (D.n_tris + 31) / 32;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
-    for (int b0 = 0; b0 < nb; b0 += blockDim.x) {
-        const int i = b0 + threadIdx.x;
-        const int v = i < nb ? sums[i] : 0;
-        __shared__ int round_total;
-        const int e = block_excl_scan(v, warp_sums, &round_total) + carry;
-        if (i < nb) sums[i] = e;
+    for (int b0 = 0; b0 < nb; b0 += 1024 * kScanItems) {
+        const int base = b0 + int(threadIdx.x) * kScanItems;
+        int v[kScanItems], run = 0;
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q) {
+            v[q] = base + q < nb ? a[base + q] : 0;
+            run += v[q];
+        }
+        int off = block_excl_scan(run, warp_sums, &round_total) + carry;
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q) {
+            if (base + q < nb) a[base + q] = off;
+            off += v[q];
+        }
         __syncthreads();
         if (threadIdx.x == 0) carry += round_total;
         __syncthreads();
     }
-    if (total && threadIdx.x == 0) *total = carry;
+    if (threadIdx.x == 0) {
+        *D.ws_total = carry;
+        *D.n_pairs = carry;
+        if (carry > D.max_pairs) atomicOr(D.status, XPBD_STATUS_PAIR_OVERFLOW);
+        *D.n_contacts = 0;
+    }
 }
 
-__global__ void __launch_bounds__(1024) k_scan_add(int* __restrict__ a, int n, const int* __restrict__ sums) {
-    const int add = sums[blockIdx.x];
-    const int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
-#pragma unroll
-    for (int q = 0; q < kScanItems; ++q)
-        if (base + q < n) a[base + q] += add;
-}
-
-void scan_excl(int* a, int n, int* total, int* scratch, cudaStream_t s) {
-    const int nb = (n + kScanBlock - 1) / kScanBlock;
-    k_scan_blocks<<<nb, 1024, 0, s>>>(a, n, scratch);
-    k_scan_sums<<<1, 1024, 0, s>>>(scratch, nb, total);
-    if (nb > 1) k_scan_add<<<nb, 1024, 0, s>>>(a, n, scratch);
-}
-
-// Radix sort of (Morton key, triangle id), 4 passes of 8 bits, in one
+// Radix sort of (Morton key, triangle id), 3 passes of 8 bits, in one
 // cooperative launch: CTA b owns the contiguous chunk [b C, (b+1) C) of the
 // pass input.  Per pass: (A) chunk histogram -> hist[b][256]; grid barrier;
 // (B) every CTA sums the histograms itself (digit totals, and the counts of
@@ -178,7 +165,8 @@ void scan_excl(int* a, int n, int* total, int* scratch, cudaStream_t s) {
 // first output slot per digit; (C) stable scatter in rounds of kSortThreads
 // keys: warps rank equal digits with __match_any_sync, per-digit prefix over
 // the warps in shared memory; grid barrier before the next pass reads.
-// Even pass count: the sorted data ends in ws_keys/ws_vals.
+// Odd pass count: the input is in ws_keys2/ws_vals2, the sorted data ends in
+// ws_keys/ws_vals.
 __device__ __forceinline__ int add_excl_over_warps(int (*wcnt)[256], int d, int run) {
     for (int ww = 0; ww < kSortThreads / 32; ++ww) {
         const int c = wcnt[ww][d];
@@ -197,12 +185,12 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, int chunk
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int beg = min(n, b * chunk), end = min(n, beg + chunk);
     int* hist = D.ws_hist;  // [G][256]
-    uint32_t* ks = D.ws_keys;
-    int32_t* vs = D.ws_vals;
-    uint32_t* kd = D.ws_keys2;
-    int32_t* vd = D.ws_vals2;
+    uint32_t* ks = D.ws_keys2;
+    int32_t* vs = D.ws_vals2;
+    uint32_t* kd = D.ws_keys;
+    int32_t* vd = D.ws_vals;
     GridBarrier bar = grid_barrier_begin(sync);
-    for (int pass = 0; pass < 4; ++pass) {
+    for (int pass = 0; pass < 3; ++pass) {
         const int shift = 8 * pass;
         // (A) chunk histogram
         if (threadIdx.x < 256) run[threadIdx.x] = 0;
@@ -263,124 +251,14 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, int chunk
             }
             __syncthreads();
         }
-        if (pass < 3) grid_barrier(bar, D.status);
+        if (pass < 2) grid_barrier(bar, D.status);
         uint32_t* tk = ks; ks = kd; kd = tk;
         int32_t* tv = vs; vs = vd; vd = tv;
     }
     grid_barrier_end(sync, bar);
 }
 
-// ---------------------------------------------------------- Karras build
-__device__ __forceinline__ int delta(const uint32_t* k, int n, int i, int j) {
-    if (j < 0 || j >= n) return -1;
-    const uint32_t a = k[i], b = k[j];
-    if (a == b) return 32 + __clz(uint32_t(i) ^ uint32_t(j));
-    return __clz(a ^ b);
-}
-
-// Box of the sorted leaves [a, b): leaf boxes at the ends, 32-leaf block boxes
-// (ws_bbox[0, nb32)) and 1024-leaf block boxes (ws_bbox[nb32, ...)) between.
-// Independent loads, no dependence on other internal nodes: the whole
-// hierarchy's boxes come out of the build launch without a bottom-up refit.
-struct Box {
-    float4 lo, hi;
-    __device__ __forceinline__ void add(const float4* p, int k) {
-        const float4 l = p[2 * k], h = p[2 * k + 1];
-        lo.x = fminf(lo.x, l.x), lo.y = fminf(lo.y, l.y), lo.z = fminf(lo.z, l.z);
-        hi.x = fmaxf(hi.x, h.x), hi.y = fmaxf(hi.y, h.y), hi.z = fmaxf(hi.z, h.z);
-    }
-};
-
-__device__ __forceinline__ void add_run(Box& bx, const float4* p, int a, int b) {
-#pragma unroll 4
-    for (int k = a; k < b; ++k) bx.add(p, k);
-}
-
-__device__ Box range_box(const XpbdDcd& D, int a, int b) {
-    const int n = D.n_tris;
-    const float4* leaves = reinterpret_cast<const float4*>(D.ws_nodes) + sorted_leaf_base(n);
-    const float4* b32 = reinterpret_cast<const float4*>(D.ws_bbox);
-    const float4* b1k = b32 + 2 * ((n + 31) / 32);
-    Box bx;
-    bx.lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-    bx.hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    if (b - a <= 64) {
-        add_run(bx, leaves, a, b);
-        return bx;
-    }
-    const int a1 = (a + 31) >> 5, e1 = b >> 5;  // whole 32-leaf blocks [a1, e1)
-    add_run(bx, leaves, a, a1 << 5);
-    add_run(bx, leaves, e1 << 5, b);
-    if (e1 - a1 <= 64) {
-        add_run(bx, b32, a1, e1);
-        return bx;
-    }
-    const int a2 = (a1 + 31) >> 5, e2 = e1 >> 5;  // whole 1024-leaf blocks [a2, e2)
-    add_run(bx, b32, a1, a2 << 5);
-    add_run(bx, b32, e2 << 5, e1);
-    add_run(bx, b1k, a2, e2);
-    return bx;
-}
-
-// Half `side` of internal node i's record: the box of the child covering
-// [lo, g] (side 0) or [g + 1, hi] (side 1), its last Morton position, its id.
-__device__ __forceinline__ void write_child(const XpbdDcd& D, int i, int side, int lo, int g, int hi) {
-    const int n = D.n_tris;
-    const int first = side ? g + 1 : lo, last = side ? hi : g;
-    const int id = (first == last) ? (n - 1 + first) : (side ? g + 1 : g);
-    const Box bx = range_box(D, first, last + 1);
-    float4* rec = reinterpret_cast<float4*>(D.ws_nodes) + 4 * int64_t(i) + 2 * side;
-    rec[0] = make_float4(bx.lo.x, bx.lo.y, bx.lo.z, __int_as_float(last));
-    rec[1] = make_float4(bx.hi.x, bx.hi.y, bx.hi.z, __int_as_float(id));
-}
-
-// Karras (2012) hierarchy over the sorted keys.  Two threads per internal
-// node i (adjacent lanes) both run its split search; thread `side` then
-// writes child `side`'s half of record i: box from the child's leaf range,
-// last Morton position, node id.  Two threads halve the range-box work per
-// thread and double the warps in flight: the launch is latency-bound.
-__global__ void k_build(XpbdDcd D) {
-    const int n = D.n_tris;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = gid >> 1, side = gid & 1;
-    if (i >= n - 1) return;
-    const uint32_t* k = D.ws_keys;
-    const int d = (delta(k, n, i, i + 1) - delta(k, n, i, i - 1)) >= 0 ? 1 : -1;
-    const int dmin = delta(k, n, i, i - d);
-    int lmax = 2;
-    while (lmax < 2 * n && delta(k, n, i, i + lmax * d) > dmin) lmax <<= 1;
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (delta(k, n, i, i + (l + t) * d) > dmin) l += t;
-    const int j = i + l * d;
-    const int dnode = delta(k, n, i, j);
-    int s = 0;
-    int t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (delta(k, n, i, i + (s + t) * d) > dnode) s += t;
-    } while (t > 1);
-    const int g = i + s * d + min(d, 0);
-    const int lo = min(i, j), hi = max(i, j);
-    if (side == 0) reinterpret_cast<int4*>(D.ws_split)[i] = make_int4(lo, g, hi, 0);
-    write_child(D, i, side, lo, g, hi);
-}
-
-// Refit-only broadphase: the hierarchy of the last rebuild (leaf range and
-// split per internal node in ws_split) over the leaves in that rebuild's
-// Morton order, boxes recomputed from the current leaf boxes.  The pair set
-// does not depend on the hierarchy, only the traversal cost does.
-__global__ void k_refit_ranges(XpbdDcd D) {
-    const int n = D.n_tris;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = gid >> 1, side = gid & 1;
-    if (i >= n - 1) return;
-    const int4 r = reinterpret_cast<const int4*>(D.ws_split)[i];
-    write_child(D, i, side, r.x, r.y, r.z);
-}
-
-// Leaves were written in triangle order; the build wants them in Morton order.  A CTA of 1024 threads covers 1024
-// consecutive leaves and also writes their 32- and 1024-leaf block boxes.
+// ---------------------------------------------------------- leaves and blocks
 __device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
@@ -393,26 +271,34 @@ __device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
     }
 }
 
-__global__ void __launch_bounds__(1024) k_permute_leaves(XpbdDcd D) {
+// Leaf records in Morton order from the current positions, and the boxes of the
+// CTA's 32- and 1024-leaf blocks.  All that a refit-only broadphase runs before
+// the traversal (the order of the last rebuild stays; the pair set does not
+// depend on it).
+__global__ void __launch_bounds__(1024) k_leaves(XpbdDcd D, const float* __restrict__ pos4) {
     __shared__ float4 s_box[32][2];
     const int n = D.n_tris;
     const int s = blockIdx.x * 1024 + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const Leaves L(D);
     float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
     if (s < n) {
         const int tri = D.ws_vals[s];
-        const float4* src = reinterpret_cast<const float4*>(D.ws_nodes) + tri_leaf_base(n);
-        float4* dst = reinterpret_cast<float4*>(D.ws_nodes) + sorted_leaf_base(n);
-        lo = src[2 * tri];
-        hi = src[2 * tri + 1];
-        dst[2 * s] = lo;
-        dst[2 * s + 1] = hi;
+        if (tri >= 0 && tri < n) {  // always, unless the sort gave up
+            const int a = D.tris[3 * tri], b = D.tris[3 * tri + 1], c = D.tris[3 * tri + 2];
+            float3 l, h;
+            tri_box(D, pos4, a, b, c, l, h);
+            lo = make_float4(l.x, l.y, l.z, __int_as_float(tri));
+            hi = make_float4(h.x, h.y, h.z, __int_as_float(D.tri_group ? D.tri_group[tri] : 0));
+            L.verts[s] = make_int4(a, b, c, 0);
+        }
+        L.lo[s] = lo;
+        L.hi[s] = hi;
     }
     warp_box(lo, hi);
-    float4* b32 = reinterpret_cast<float4*>(D.ws_bbox);
     if (lane == 0 && s < n) {
-        b32[2 * (s >> 5)] = lo;
-        b32[2 * (s >> 5) + 1] = hi;
+        L.b32[2 * (s >> 5)] = lo;
+        L.b32[2 * (s >> 5) + 1] = hi;
     }
     if (lane == 0) {
         s_box[w][0] = lo;
@@ -424,9 +310,8 @@ __global__ void __launch_bounds__(1024) k_permute_leaves(XpbdDcd D) {
         hi = s_box[lane][1];
         warp_box(lo, hi);
         if (lane == 0) {
-            float4* b1k = b32 + 2 * ((n + 31) / 32);
-            b1k[2 * blockIdx.x] = lo;
-            b1k[2 * blockIdx.x + 1] = hi;
+            L.b1k[2 * blockIdx.x] = lo;
+            L.b1k[2 * blockIdx.x + 1] = hi;
         }
     }
 }
@@ -436,115 +321,125 @@ __device__ __forceinline__ bool overlap(float4 alo, float4 ahi, float4 blo, floa
     return !(alo.x > bhi.x || blo.x > ahi.x || alo.y > bhi.y || blo.y > ahi.y || alo.z > bhi.z || blo.z > ahi.z);
 }
 
-// broadphase_find_pairs_bvh_kernel rules (udcf/kernel.py:937-981): j > i,
-// static-static never, movable-self only when allowed and sharing no vertex.
-__device__ __forceinline__ bool pair_ok(const XpbdDcd& D, int i, int j) {
-    if (j <= i) return false;
-    const int gi = D.tri_group ? D.tri_group[i] : 0, gj = D.tri_group ? D.tri_group[j] : 0;
-    if (gi == 1 && gj == 1) return false;
-    if (gi == 0 && gj == 0) {
-        if (!D.allow_self) return false;
-        const int a0 = D.tris[3 * i], a1 = D.tris[3 * i + 1], a2 = D.tris[3 * i + 2];
-        const int b0 = D.tris[3 * j], b1 = D.tris[3 * j + 1], b2 = D.tris[3 * j + 2];
-        if (a0 == b0 || a0 == b1 || a0 == b2 || a1 == b0 || a1 == b1 || a1 == b2 || a2 == b0 || a2 == b1 || a2 == b2)
-            return false;
-    }
-    return true;
+__device__ __forceinline__ float4 shfl4(float4 v, int src) {
+    return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                       __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
 
-// Thread t queries the triangle at Morton position t against the leaves at
-// later positions only: every unordered overlapping pair is met once, by the
-// query that comes first in Morton order, and subtrees whose last position
-// (kept in the node's lo.w) is <= t are skipped whole.  A warp's queries are
-// spatially close and walk similar paths.  Both children are tested before
-// descending; one stack entry per level with two live children.
-// The counting pass keeps the first kSlots partners in ws_slots; the fill
-// pass copies those and re-traverses only queries with more partners.
-// Pairs are written as (min, max) triangle id, grouped by query position.
-__device__ __forceinline__ bool live(const float4& qlo, const float4& qhi, const float4& lo, const float4& hi, int t) {
-    return __float_as_int(lo.w) > t && overlap(qlo, qhi, lo, hi);
-}
-
-template <bool FILL>
-__device__ __forceinline__ void emit_leaf(const XpbdDcd& D, int i, int leaf_pos, int t, int& cnt, int& out) {
-    const int j = D.ws_vals[leaf_pos];
-    const int a = min(i, j), b = max(i, j);
-    if (!pair_ok(D, a, b)) return;
-    if (FILL) {
-        if (out < D.max_pairs) reinterpret_cast<int2*>(D.pairs)[out] = make_int2(a, b);
-        ++out;
-    } else {
-        if (cnt < kSlots) D.ws_slots[int64_t(cnt) * D.n_tris + t] = j;
-        ++cnt;
+// A warp lists the pairs of the 32 triangles at Morton positions 32 qb + lane
+// with the triangles at later positions (every unordered pair is met once).
+// Blocks are found with the common box, 32 per test, and kept only for the
+// lanes whose own box touches them: 32 neighbours that straddle a jump of the
+// Morton curve have a common box as large as the scene, yet each of them
+// touches a dozen 32-leaf blocks at most.  In a block that is kept, each of
+// those lanes' boxes in turn meets all 32 leaves, one per lane, so the work is
+// the number of (triangle, block) contacts, 3.5 per triangle of a body, however
+// the common box lies (a loop over the leaves that touch the common box took
+// 1620 us for 105k triangles in the warps at such jumps).
+// emit(src, hits, hit, j): for query lane src, in ascending partner position,
+// the lanes of the ballot `hits` pair it with their triangle j; `on`: the lanes
+// that take part as queries.  Pair rules of broadphase_find_pairs_bvh_kernel
+// (udcf/kernel.py:937-981): static-static never, movable-self only when allowed
+// and sharing no vertex.
+template <class Emit>
+__device__ __forceinline__ void walk_blocks(const XpbdDcd& D, int qb, bool on, Emit emit) {
+    const Leaves L(D);
+    const int n = D.n_tris, nb = (n + 31) / 32, nk = (n + 1023) / 1024;
+    const int lane = threadIdx.x & 31, t = 32 * qb + lane;
+    const float4 ulo = L.b32[2 * qb], uhi = L.b32[2 * qb + 1];
+    float4 qlo = make_float4(0.f, 0.f, 0.f, 0.f), qhi = qlo;
+    int4 qv = make_int4(-1, -1, -1, 0);
+    on = on && t < n;
+    if (on) {
+        qlo = L.lo[t];
+        qhi = L.hi[t];
+        qv = L.verts[t];
     }
-}
-
-template <bool FILL>
-__global__ void __launch_bounds__(128) k_traverse(XpbdDcd D) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = D.n_tris;
-    if (t >= n) return;
-    if (*D.status & XPBD_STATUS_BARRIER_TIMEOUT) return;  // the sort gave up: no valid tree
-    const int i = D.ws_vals[t];
-    int cnt = 0, out = 0;
-    if (FILL) {
-        out = D.ws_count[t];
-        const int end = t + 1 < n ? D.ws_count[t + 1] : *D.ws_total;
-        const int c = end - out;
-        if (c <= kSlots) {
-            for (int k = 0; k < c; ++k, ++out) {
-                if (out >= D.max_pairs) break;
-                const int j = D.ws_slots[int64_t(k) * n + t];
-                reinterpret_cast<int2*>(D.pairs)[out] = make_int2(min(i, j), max(i, j));
-            }
-            return;
-        }
-    }
-    if (n > 1) {
-        const float4* recs = reinterpret_cast<const float4*>(D.ws_nodes);
-        const float4* tri_box = recs + tri_leaf_base(n);
-        const float4 qlo = tri_box[2 * i], qhi = tri_box[2 * i + 1];
-        int stack[kStack];
-        int sp = 0;
-        int node = 0;  // the root (its own box is never needed: its record tests both children)
-        for (int visits = 0;; ++visits) {
-            if (visits >= n) {  // more internal nodes than the tree has: not a tree
-                atomicOr(D.status, XPBD_STATUS_STACK_OVERFLOW);
-                break;
-            }
-            const float4* r = recs + 4 * int64_t(node);
-            const float4 alo = r[0], ahi = r[1], blo = r[2], bhi = r[3];
-            const int ca = __float_as_int(ahi.w), cb = __float_as_int(bhi.w);
-            const bool la = live(qlo, qhi, alo, ahi, t);
-            const bool lb = live(qlo, qhi, blo, bhi, t);
-            const bool da = la && ca < n - 1, db = lb && cb < n - 1;  // internal children to descend
-            if (la && !da) emit_leaf<FILL>(D, i, ca - (n - 1), t, cnt, out);
-            if (lb && !db) emit_leaf<FILL>(D, i, cb - (n - 1), t, cnt, out);
-            if (da && db) {
-                if (sp >= kStack) {
-                    atomicOr(D.status, XPBD_STATUS_STACK_OVERFLOW);
-                    break;
+    for (int k0 = qb >> 5; k0 < nk; k0 += 32) {
+        const int k = min(k0 + lane, nk - 1);
+        const float4 klo = L.b1k[2 * k], khi = L.b1k[2 * k + 1];
+        unsigned mk = __ballot_sync(0xffffffffu, k0 + lane < nk && overlap(ulo, uhi, klo, khi));
+        for (; mk; mk &= mk - 1) {
+            const int ks = __ffs(mk) - 1, c0 = 32 * (k0 + ks), c = min(c0 + lane, nb - 1);
+            const float4 kl = shfl4(klo, ks), kh = shfl4(khi, ks);
+            if (!__any_sync(0xffffffffu, on && overlap(qlo, qhi, kl, kh))) continue;
+            const float4 clo = L.b32[2 * c], chi = L.b32[2 * c + 1];
+            unsigned mc = __ballot_sync(0xffffffffu, c0 + lane >= qb && c0 + lane < nb && overlap(ulo, uhi, clo, chi));
+            for (; mc; mc &= mc - 1) {
+                const int cs = __ffs(mc) - 1;
+                const float4 cl = shfl4(clo, cs), ch = shfl4(chi, cs);
+                unsigned mq = __ballot_sync(0xffffffffu, on && overlap(qlo, qhi, cl, ch));
+                if (!mq) continue;
+                const int p = 32 * (c0 + cs) + lane, pc = min(p, n - 1);
+                const float4 lo = L.lo[pc], hi = L.hi[pc];
+                for (; mq; mq &= mq - 1) {
+                    const int src = __ffs(mq) - 1;
+                    const float4 alo = shfl4(qlo, src), ahi = shfl4(qhi, src);
+                    bool hit = p < n && p > 32 * qb + src && overlap(alo, ahi, lo, hi);
+                    if (!__any_sync(0xffffffffu, hit)) continue;
+                    const int g = __float_as_int(hi.w), ag = __float_as_int(ahi.w);
+                    const int a = __shfl_sync(0xffffffffu, qv.x, src), b = __shfl_sync(0xffffffffu, qv.y, src),
+                              d = __shfl_sync(0xffffffffu, qv.z, src);
+                    if (g == 1 && ag == 1) hit = false;
+                    if (hit && g == 0 && ag == 0) {
+                        const int4 v = L.verts[pc];
+                        hit = D.allow_self && !(v.x == a || v.x == b || v.x == d || v.y == a || v.y == b || v.y == d ||
+                                                v.z == a || v.z == b || v.z == d);
+                    }
+                    const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                    if (hits) emit(src, hits, hit, __float_as_int(lo.w));
                 }
-                stack[sp++] = cb;
-                node = ca;
-            } else if (da || db) {
-                node = da ? ca : cb;
-            } else {
-                if (sp == 0) break;
-                node = stack[--sp];
             }
         }
     }
-    if (!FILL) D.ws_count[t] = cnt;
 }
 
-__global__ void k_pairs_total(XpbdDcd D) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const int tot = *D.ws_total;
-        *D.n_pairs = tot;
-        if (tot > D.max_pairs) atomicOr(D.status, XPBD_STATUS_PAIR_OVERFLOW);
-        *D.n_contacts = 0;
+// Counting pass: pairs per query (ws_count) and per block of 32 (ws_keys2); a
+// query's first kSlots partners are kept for the fill pass.
+__global__ void __launch_bounds__(128) k_count_pairs(XpbdDcd D) {
+    const int qb = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int n = D.n_tris, t = 32 * qb + lane;
+    if (32 * qb >= n) return;
+    int cnt = 0;
+    if (!(*D.status & XPBD_STATUS_BARRIER_TIMEOUT))  // else the sort gave up: no valid order, no pairs
+        walk_blocks(D, qb, true, [&](int src, unsigned hits, bool hit, int j) {
+            const int slot = __shfl_sync(0xffffffffu, cnt, src) + __popc(hits & ((1u << lane) - 1u));
+            if (hit && slot < kSlots) D.ws_slots[int64_t(slot) * n + 32 * qb + src] = j;
+            if (lane == src) cnt += __popc(hits);
+        });
+    if (t < n) D.ws_count[t] = cnt;
+    const int total = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) reinterpret_cast<int*>(D.ws_keys2)[qb] = total;
+}
+
+// Fill pass: pairs as (min, max) triangle id, grouped by query position; only
+// queries with more than kSlots partners walk again.
+__global__ void __launch_bounds__(128) k_fill_pairs(XpbdDcd D) {
+    const int qb = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int n = D.n_tris, t = 32 * qb + lane;
+    if (32 * qb >= n) return;
+    const int c = t < n ? D.ws_count[t] : 0;
+    if (!__any_sync(0xffffffffu, c != 0)) return;
+    int out = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, out, o);
+        if (lane >= o) out += y;
     }
+    out += reinterpret_cast<const int*>(D.ws_keys2)[qb] - c;
+    const int i = c ? D.ws_vals[t] : 0;
+    int2* pairs = reinterpret_cast<int2*>(D.pairs);
+    for (int k = 0; k < c && c <= kSlots; ++k) {
+        const int j = D.ws_slots[int64_t(k) * n + t];
+        if (out + k < D.max_pairs) pairs[out + k] = make_int2(min(i, j), max(i, j));
+    }
+    const bool again = c > kSlots;
+    if (__any_sync(0xffffffffu, again))
+        walk_blocks(D, qb, again, [&](int src, unsigned hits, bool hit, int j) {
+            const int k = __shfl_sync(0xffffffffu, out, src) + __popc(hits & ((1u << lane) - 1u));
+            const int is = __shfl_sync(0xffffffffu, i, src);
+            if (hit && k < D.max_pairs) pairs[k] = make_int2(min(is, j), max(is, j));
+            if (lane == src) out += __popc(hits);
+        });
 }
 
 // ------------------------------------------------------------ narrowphase
@@ -596,10 +491,12 @@ __device__ __forceinline__ bool gen_t(float3 N, float3 v0, float3 v1, float3 v2,
     return true;
 }
 
-__global__ void k_narrow(XpbdDcd D, const float* __restrict__ pos4) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int np = min(*D.n_pairs, D.max_pairs);
-    if (k >= np) return;
+__device__ __forceinline__ void respond(const XpbdDcd& D, const float* pos4, int4 cu, int4 cl, float4 f0, float4 f1,
+                                        float4 f2);
+
+// One pair; a contact is listed and responded to at once (the responses go to
+// the accumulator, no position moves before k_dcd_apply).
+__device__ __forceinline__ void narrow_pair(const XpbdDcd& D, const float* __restrict__ pos4, int k) {
     const int ta = D.pairs[2 * k], tb = D.pairs[2 * k + 1];
     const float3 q00 = f3(ld4(pos4, D.tris[3 * ta])), q01 = f3(ld4(pos4, D.tris[3 * ta + 1])),
                  q02 = f3(ld4(pos4, D.tris[3 * ta + 2]));
@@ -704,26 +601,31 @@ __global__ void k_narrow(XpbdDcd D, const float* __restrict__ pos4) {
     const bool first = C1 < C2;  // tie -> C2 branch
     const int tc = first ? ta : tb, tl = first ? tb : ta;
     int4* cid = reinterpret_cast<int4*>(D.c_ids);
-    cid[2 * slot] = make_int4(D.tris[3 * tc], D.tris[3 * tc + 1], D.tris[3 * tc + 2], k);
-    cid[2 * slot + 1] = make_int4(D.tris[3 * tl], D.tris[3 * tl + 1], D.tris[3 * tl + 2], 0);
+    const int4 cu = make_int4(D.tris[3 * tc], D.tris[3 * tc + 1], D.tris[3 * tc + 2], k);
+    const int4 cl = make_int4(D.tris[3 * tl], D.tris[3 * tl + 1], D.tris[3 * tl + 2], 0);
+    cid[2 * slot] = cu;
+    cid[2 * slot + 1] = cl;
     float4* cf = reinterpret_cast<float4*>(D.c_data);
     const float3 n = first ? N2 : N1;
     const float3 bb1 = first ? b1 : b3, bb2 = first ? b2 : b4;
-    cf[3 * slot] = make_float4(n.x, n.y, n.z, first ? C1 : C2);
-    cf[3 * slot + 1] = make_float4(bb1.x, bb1.y, bb1.z, C1);
-    cf[3 * slot + 2] = make_float4(bb2.x, bb2.y, bb2.z, C2);
+    const float4 f0 = make_float4(n.x, n.y, n.z, first ? C1 : C2), f1 = make_float4(bb1.x, bb1.y, bb1.z, C1),
+                 f2 = make_float4(bb2.x, bb2.y, bb2.z, C2);
+    cf[3 * slot] = f0;
+    cf[3 * slot + 1] = f1;
+    cf[3 * slot + 2] = f2;
+    respond(D, pos4, cu, cl, f0, f1, f2);
+}
+
+// The pair count is known on the device only: a grid that fills the GPU strides
+// over it (a thread per possible pair was 16,384 CTAs, 17 us to find 31k pairs).
+__global__ void __launch_bounds__(256) k_narrow(XpbdDcd D, const float* __restrict__ pos4) {
+    const int np = min(*D.n_pairs, D.max_pairs);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) narrow_pair(D, pos4, k);
 }
 
 // respond_kernel (udcf/kernel.py:713-806)
-__global__ void k_respond(XpbdDcd D, const float* __restrict__ pos4) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nc = min(*D.n_contacts, D.max_contacts);
-    if (k >= nc) return;
-    const int4 cu = reinterpret_cast<const int4*>(D.c_ids)[2 * k];
-    const int4 cl = reinterpret_cast<const int4*>(D.c_ids)[2 * k + 1];
-    const float4 f0 = reinterpret_cast<const float4*>(D.c_data)[3 * k];
-    const float4 f1 = reinterpret_cast<const float4*>(D.c_data)[3 * k + 1];
-    const float4 f2 = reinterpret_cast<const float4*>(D.c_data)[3 * k + 2];
+__device__ __forceinline__ void respond(const XpbdDcd& D, const float* pos4, int4 cu, int4 cl, float4 f0, float4 f1,
+                                        float4 f2) {
     float pen = f0.w;
     if (D.max_push > 0.f && pen > D.max_push) pen = D.max_push;
     float C = pen * D.multiplier;
@@ -766,7 +668,7 @@ __global__ void k_respond(XpbdDcd D, const float* __restrict__ pos4) {
 // apply_kernel (udcf/kernel.py:809-822), clearing the accumulator it reads
 __global__ void k_dcd_apply(XpbdDcd D, float* pos4) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.n_verts) return;
+    if (i >= D.n_verts || *D.n_contacts == 0) return;
     float4* acc = reinterpret_cast<float4*>(D.dP);
     const float4 a = acc[i];
     if (a.w > 0.f) {
@@ -785,14 +687,8 @@ __global__ void k_dcd_apply(XpbdDcd D, float* pos4) {
     }
 }
 
-__global__ void k_copy4(const float4* __restrict__ src, float4* __restrict__ dst, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[i];
-}
-
 // Sort CTAs: one per kSortThreads keys, at most the co-resident count.
 int64_t hist_words(int n) { return int64_t(256) * ((n + kSortThreads - 1) / kSortThreads); }
-int64_t scan_words(int n) { return (n + kScanBlock - 1) / kScanBlock; }
 
 int launch_sort(const XpbdDcd* D, uint32_t* sync, cudaStream_t s) {
     static int slots[64] = {};
@@ -843,14 +739,13 @@ extern "C" {
 
 int xpbd_dcd_workspace_query(int32_t n_tris, XpbdDcdWorkspaceSizes* out) {
     if (n_tris <= 0 || !out) return fail(XPBD_ERR_ARG, "xpbd_dcd_workspace_query: bad arguments");
-    out->nodes_floats = (tri_leaf_base(n_tris) + 2 * int64_t(n_tris)) * 4;  // records, leaves x2
+    out->nodes_floats = int64_t(12) * n_tris;  // leaf records
     out->keys = n_tris;
-    // sort histograms [CTAs][256], the count scan's block sums, the sort's barrier words
-    out->hist = hist_words(n_tris) + scan_words(n_tris) + 4;
+    out->hist = hist_words(n_tris) + 4;  // sort histograms [CTAs][256], the sort's barrier words
     out->bbox_floats = int64_t(8) * ((n_tris + 31) / 32 + (n_tris + 1023) / 1024);  // 32- and 1024-leaf block boxes
     out->count = n_tris;
     out->slots = int64_t(kSlots) * n_tris;
-    out->split = int64_t(4) * (n_tris > 1 ? n_tris - 1 : 1);
+    out->split = 4;  // unused
     return XPBD_OK;
 }
 
@@ -860,25 +755,13 @@ int xpbd_dcd_broadphase(const XpbdDcd* D, const float* pos4, int32_t snapshot_pr
     if (!pos4 || !aligned16(pos4)) return fail(XPBD_ERR_ARG, "xpbd_dcd_broadphase: pos4");
     cudaStream_t s = (cudaStream_t)stream;
     const int n = D->n_tris;
-    if (snapshot_prev)
-        k_copy4<<<(D->n_verts + 255) / 256, 256, 0, s>>>(reinterpret_cast<const float4*>(pos4),
-                                                          reinterpret_cast<float4*>(D->x_prev), D->n_verts);
-    int* scan_scratch = D->ws_hist + hist_words(n);
-    if (D->refit_only) {
-        k_tri_aabb<false><<<(n + 255) / 256, 256, 0, s>>>(*D, pos4);
-        k_permute_leaves<<<(n + 1023) / 1024, 1024, 0, s>>>(*D);
-        if (n > 1) k_refit_ranges<<<(2 * (n - 1) + 255) / 256, 256, 0, s>>>(*D);
-    } else {
-        k_tri_aabb<true><<<(n + 255) / 256, 256, 0, s>>>(*D, pos4);
-        uint32_t* sort_sync = reinterpret_cast<uint32_t*>(scan_scratch + scan_words(n));
-        if ((rc = launch_sort(D, sort_sync, s))) return rc;
-        k_permute_leaves<<<(n + 1023) / 1024, 1024, 0, s>>>(*D);
-        if (n > 1) k_build<<<(2 * (n - 1) + 255) / 256, 256, 0, s>>>(*D);
-    }
-    k_traverse<false><<<(n + 127) / 128, 128, 0, s>>>(*D);
-    scan_excl(D->ws_count, n, D->ws_total, scan_scratch, s);
-    k_traverse<true><<<(n + 127) / 128, 128, 0, s>>>(*D);
-    k_pairs_total<<<1, 32, 0, s>>>(*D);
+    const int rows = std::max(D->refit_only ? 0 : n, snapshot_prev ? D->n_verts : 0);
+    if (rows > 0) k_tri_keys<<<(rows + 255) / 256, 256, 0, s>>>(*D, pos4, D->refit_only ? 0 : 1, snapshot_prev);
+    if (!D->refit_only && (rc = launch_sort(D, reinterpret_cast<uint32_t*>(D->ws_hist + hist_words(n)), s))) return rc;
+    k_leaves<<<(n + 1023) / 1024, 1024, 0, s>>>(*D, pos4);
+    k_count_pairs<<<(n + 127) / 128, 128, 0, s>>>(*D);
+    k_scan_pairs<<<1, 1024, 0, s>>>(*D);
+    k_fill_pairs<<<(n + 127) / 128, 128, 0, s>>>(*D);
     return cuda_check("xpbd_dcd_broadphase");
 }
 
@@ -888,8 +771,7 @@ int xpbd_dcd_narrow_respond(const XpbdDcd* D, float* pos4, xpbd_stream_t stream)
     if (!pos4 || !aligned16(pos4)) return fail(XPBD_ERR_ARG, "xpbd_dcd_narrow_respond: pos4");
     cudaStream_t s = (cudaStream_t)stream;
     cudaMemsetAsync(D->n_contacts, 0, sizeof(int32_t), s);
-    k_narrow<<<(D->max_pairs + 255) / 256, 256, 0, s>>>(*D, pos4);
-    k_respond<<<(D->max_contacts + 255) / 256, 256, 0, s>>>(*D, pos4);
+    k_narrow<<<std::min((D->max_pairs + 255) / 256, kNarrowCtas), 256, 0, s>>>(*D, pos4);
     k_dcd_apply<<<(D->n_verts + 255) / 256, 256, 0, s>>>(*D, pos4);
     return cuda_check("xpbd_dcd_narrow_respond");
 }

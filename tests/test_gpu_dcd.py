@@ -151,3 +151,22 @@ def test_penetration_resolves_on_gpu():
     s.synchronize()
     assert buf.counters()["n_pairs"] == 1
     assert -float(p.cpu().numpy()[0:3, 1].min()) < depth0 * 0.5
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1023, 1024, 1025, 4200])
+def test_pairs_at_block_edges(n):
+    """Triangle counts around the 32- and 1024-leaf blocks, clustered so that
+    many queries have more partners than the 16 the counting pass keeps."""
+    rng = np.random.default_rng(n)
+    cen = (rng.random((n, 3)) ** 3).astype(np.float32)
+    verts = (cen[:, None, :] + rng.normal(scale=0.03, size=(n, 3, 3)).astype(np.float32)).reshape(-1, 3)
+    p4 = np.ones((3 * n, 4), np.float32)
+    p4[:, :3] = verts
+    tris = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    prm = UdcfParams(allow_self=True, thickness=0.001, max_pairs=1 << 21, max_contacts=1 << 18)
+    a, b = _run(tris, p4, prm), _run(tris, p4, prm)
+    ref, _ = O.dcd_pairs(tris, p4, thickness=prm.thickness, allow_self=True)
+    assert a["counters"]["status"] == 0
+    got = a["pairs"][np.lexsort((a["pairs"][:, 1], a["pairs"][:, 0]))]
+    np.testing.assert_array_equal(got, ref)
+    np.testing.assert_array_equal(a["pairs"], b["pairs"])
