@@ -45,7 +45,7 @@ __device__ __forceinline__ void sdf_push(const XpbdSdf& S, float4& p) {
     if (!(gl > 1e-12f)) return;
     const float err = phi - S.contact_offset;
     if (err < 0.f && (S.max_push <= 0.f || -err <= S.max_push)) {
-        const float3 n = __fdividef(1.f, gl) * gr;
+        const float3 n = gr / gl;
         p.x -= n.x * err;
         p.y -= n.y * err;
         p.z -= n.z * err;
@@ -60,10 +60,9 @@ __device__ __forceinline__ void vertex_step_regs(const XpbdParams& prm, const Xp
     const float dt = prm.dt;
     if (ops & XPBD_OP_SDF) sdf_push(S, p);
     if (ops & XPBD_OP_VELOCITY) {
-        const float inv_dt = 1.f / dt;
-        v.x = (p.x - q.x) * inv_dt;
-        v.y = (p.y - q.y) * inv_dt;
-        v.z = (p.z - q.z) * inv_dt;
+        v.x = (p.x - q.x) / dt;
+        v.y = (p.y - q.y) / dt;
+        v.z = (p.z - q.z) / dt;
     }
     if (ops & XPBD_OP_PREDICT) {
         q = make_float4(p.x, p.y, p.z, 0.f);
