@@ -479,7 +479,7 @@ typedef struct XpbdDcd {
     float multiplier;         /* collisionConstraintMultiplier (1.01) */
     float friction_static, friction_dynamic;
     float max_push;           /* > 0: clamp contact depth (UdcfParams.max_push) */
-    float box_lo[3], box_hi[3]; /* Morton quantisation box (centres outside are clamped) */
+    float box_lo[3], box_hi[3]; /* Hilbert-curve quantisation box (centres outside are clamped) */
     int32_t* pairs;           /* [max_pairs][2] (i, j > i), deterministic order; 16-byte aligned */
     int32_t* n_pairs;         /* [1] candidate pairs found (may exceed max_pairs) */
     int32_t* n_contacts;      /* [1] contacts found (may exceed max_contacts) */
@@ -488,19 +488,19 @@ typedef struct XpbdDcd {
     float* x_prev;            /* [n_verts][4] positions at the broadphase (friction reference) */
     float* dP;                /* [n_verts][4] response accumulator, zero between calls */
     int32_t* status;          /* [1] XPBD_STATUS_* bits */
-    float* ws_nodes;          /* workspace: leaf records (box, id, group, vertices) in Morton order */
-    uint32_t* ws_keys;        /* [n_tris] Morton keys (sorted in place) */
-    int32_t* ws_vals;         /* [n_tris] triangle ids in Morton order */
+    float* ws_nodes;          /* workspace: leaf records (box, id, group, vertices) in curve order */
+    uint32_t* ws_keys;        /* [n_tris] curve keys (sorted in place) */
+    int32_t* ws_vals;         /* [n_tris] triangle ids in curve order */
     uint32_t* ws_keys2;       /* [n_tris] sort ping-pong, then pairs per 32 queries and their offsets */
     int32_t* ws_vals2;        /* [n_tris] */
     int32_t* ws_hist;         /* radix histograms and the sort's four grid barrier words (its last
                                  four entries); zero before the first call */
-    float* ws_bbox;           /* boxes of 32- and 1024-leaf Morton blocks (2 float4 each) */
-    int32_t* ws_count;        /* [n_tris] pairs per Morton position */
+    float* ws_bbox;           /* boxes of 32- and 1024-leaf curve blocks (2 float4 each) */
+    int32_t* ws_count;        /* [n_tris] pairs per curve position */
     int32_t* ws_total;        /* [1] */
     int32_t* ws_slots;        /* [16][n_tris] first partners of each query (counting pass) */
     int32_t* ws_split;        /* unused (16-byte aligned, not null) */
-    int32_t refit_only;       /* 1: keep the Morton order of the last rebuild on this workspace and
+    int32_t refit_only;       /* 1: keep the curve order of the last rebuild on this workspace and
                                  recompute the boxes only (same pair set; no sort).  Needs one earlier
                                  call with 0. */
 } XpbdDcd;
@@ -512,9 +512,9 @@ typedef struct XpbdDcdWorkspaceSizes {
 
 int xpbd_dcd_workspace_query(int32_t n_tris, XpbdDcdWorkspaceSizes* out);
 
-/* AABBs in Morton order with the boxes of 32- and 1024-leaf blocks, and the
- * candidate pair list (grouped by the pair's first triangle in Morton order,
- * partners in Morton order); snapshot_prev != 0 first copies pos4 to x_prev
+/* AABBs in curve order with the boxes of 32- and 1024-leaf blocks, and the
+ * candidate pair list (grouped by the pair's first triangle in curve order,
+ * partners in curve order); snapshot_prev != 0 first copies pos4 to x_prev
  * (UdcfDcdCollider.solve with i_iter == 0, udcf/solver.py:365-382). */
 int xpbd_dcd_broadphase(const XpbdDcd* dcd, const float* pos4, int32_t snapshot_prev, xpbd_stream_t stream);
 

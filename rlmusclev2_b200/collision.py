@@ -142,7 +142,7 @@ class UdcfParams:
     gauss_seidel: bool = False
     max_push: float = 0.0
     use_bvh: bool = True
-    # Library-specific: rebuild the Morton order every n-th broadphase and only
+    # Library-specific: rebuild the curve order every n-th broadphase and only
     # recompute the boxes in between.  1 = the reference's
     # per-broadphase rebuild; the pair set is the same for any n.
     bvh_rebuild_every: int = 1
@@ -202,7 +202,7 @@ class DcdBuffers:
         self.d = d
 
     def broadphase(self, pos4: torch.Tensor, snapshot_prev: bool, stream, refit_only: bool = False) -> None:
-        """Boxes and pair list; ``refit_only`` keeps the last rebuild's Morton
+        """Boxes and pair list; ``refit_only`` keeps the last rebuild's curve
         order (the first call always rebuilds)."""
         self.d.refit_only = int(bool(refit_only) and self._built)
         capi.check(self.lib.xpbd_dcd_broadphase(C.byref(self.d), C.c_void_p(pos4.data_ptr()), int(snapshot_prev),

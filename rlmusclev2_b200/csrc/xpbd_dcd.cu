@@ -1,18 +1,20 @@
 // Triangle-triangle discrete collision detection (DCD) for sm_100a.
 //
-// Broadphase: 24-bit Morton codes of the triangles' padded boxes, a stable LSD
-// radix sort (8-bit digits, per-warp ranking with __match_any_sync), the boxes
-// in Morton order together with those of every 32 and every 1024 consecutive
-// leaves, and a block traversal: a warp takes 32 consecutive triangles and
-// walks down from the 1024-leaf blocks that their boxes touch to 32-leaf blocks,
-// and each triangle meets the 32 leaves of a block at once.  Two passes (count,
-// scan, fill) list the pairs in a deterministic order, by query and partner
-// position.
+// Broadphase: 24-bit Hilbert-curve codes of the triangles' padded boxes, a
+// stable LSD radix sort (8-bit digits, per-warp ranking with
+// __match_any_sync), the boxes in that order together with those of every 32
+// and every 1024 consecutive leaves, and a block traversal: a warp takes 32
+// consecutive triangles and walks down from the 1024-leaf blocks that their
+// boxes touch to 32-leaf blocks, and each triangle meets the 32 leaves of a
+// block at once.  Two passes (count, scan, fill) list the pairs in a
+// deterministic order, by query and partner position.
 //
 // A binary tree (Karras' construction, a query per thread) needed a build
 // launch of 32 us and left 11 of 32 lanes active on chains of dependent node
-// loads: 70 us for the counting pass of 105k triangles, the block traversal
-// takes 51 us, most of it in the warps at jumps of the curve.
+// loads: 70 us for the counting pass of 105k triangles.  The block traversal
+// takes 46 us (692k box pairs in 294k (triangle, block) tests of about 50
+// instructions; two queries at a time, half the queries a warp or up to twice
+// the resident warps all took 46 to 51 us).
 //
 // Narrowphase / response / apply restate the reference's UDCF kernels
 // (collision/udcf/kernel.py:164-474, 713-822): Moller interval rejection,
@@ -39,7 +41,7 @@ constexpr float kThresh = 1.0e-5f;  // udcf/kernel.py:40 THRESH
 
 __device__ __forceinline__ float4 ld4(const float* p, int i) { return reinterpret_cast<const float4*>(p)[i]; }
 
-// ws_nodes: three float4 arrays of the leaves in Morton order: box lo (w: the
+// ws_nodes: three float4 arrays of the leaves in curve order: box lo (w: the
 // triangle id), box hi (w: its group), vertex ids.  ws_bbox: boxes (lo, hi) of
 // the 32-leaf blocks, then of the 1024-leaf blocks.  ws_keys2 (free after the
 // sort): pairs per 32-query block, then their offsets.
@@ -75,7 +77,35 @@ __device__ __forceinline__ void tri_box(const XpbdDcd& D, const float* pos4, int
                      fmaxf(fmaxf(pa.z, pb.z), pc.z) + t);
 }
 
-// Morton keys into the buffers the first of the sort's three passes reads (8
+// Position along the Hilbert curve through the 256^3 grid (J. Skilling,
+// "Programming the Hilbert curve", 2004: undo the excess rotations from the top
+// bit down, then Gray-decode).  Against Morton order, consecutive cells always
+// touch, so no 32 neighbours straddle the scene: of the 3,288 leaf blocks of a
+// 105k-triangle body the common box of 32 queries touches 126 at most instead
+// of 531, 8.5 on average instead of 11.4, for about 90 more integer operations
+// a key.
+__device__ __forceinline__ uint32_t hilbert24(uint32_t x, uint32_t y, uint32_t z) {
+#pragma unroll
+    for (uint32_t q = 128u; q > 1u; q >>= 1) {
+        const uint32_t p = q - 1u;
+        if (x & q) x ^= p;
+        uint32_t t = (x ^ y) & p;
+        if (y & q) x ^= p;
+        else { x ^= t; y ^= t; }
+        t = (x ^ z) & p;
+        if (z & q) x ^= p;
+        else { x ^= t; z ^= t; }
+    }
+    y ^= x;
+    z ^= y;
+    uint32_t t = 0;
+#pragma unroll
+    for (uint32_t q = 128u; q > 1u; q >>= 1)
+        if (z & q) t ^= q - 1u;
+    return spread10(x ^ t) << 2 | spread10(y ^ t) << 1 | spread10(z ^ t);
+}
+
+// Curve keys into the buffers the first of the sort's three passes reads (8
 // bits per axis: cells of 3.5 mm on the 0.9-m body, about half a triangle; the
 // order only decides how tight the leaf blocks are), and the snapshot of the
 // positions when asked for.
@@ -86,15 +116,13 @@ __global__ void k_tri_keys(XpbdDcd D, const float* __restrict__ pos4, int keys, 
     float3 lo, hi;
     tri_box(D, pos4, D.tris[3 * i], D.tris[3 * i + 1], D.tris[3 * i + 2], lo, hi);
     const float q[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
-    uint32_t code = 0;
+    uint32_t u[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float ext = fmaxf(D.box_hi[k] - D.box_lo[k], 1e-30f);
-        float u = (q[k] - D.box_lo[k]) / ext * 255.f;
-        u = fminf(fmaxf(u, 0.f), 255.f);
-        code |= spread10(uint32_t(u)) << k;
+        u[k] = uint32_t(fminf(fmaxf((q[k] - D.box_lo[k]) / ext * 255.f, 0.f), 255.f));
     }
-    D.ws_keys2[i] = code;
+    D.ws_keys2[i] = hilbert24(u[0], u[1], u[2]);
     D.ws_vals2[i] = i;
 }
 
@@ -157,7 +185,7 @@ __global__ void __launch_bounds__(1024) k_scan_pairs(XpbdDcd D) {
     }
 }
 
-// Radix sort of (Morton key, triangle id), 3 passes of 8 bits, in one
+// Radix sort of (curve key, triangle id), 3 passes of 8 bits, in one
 // cooperative launch: CTA b owns the contiguous chunk [b C, (b+1) C) of the
 // pass input.  Per pass: (A) chunk histogram -> hist[b][256]; grid barrier;
 // (B) every CTA sums the histograms itself (digit totals, and the counts of
@@ -271,7 +299,7 @@ __device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
     }
 }
 
-// Leaf records in Morton order from the current positions, and the boxes of the
+// Leaf records in curve order from the current positions, and the boxes of the
 // CTA's 32- and 1024-leaf blocks.  All that a refit-only broadphase runs before
 // the traversal (the order of the last rebuild stays; the pair set does not
 // depend on it).
@@ -326,35 +354,40 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
                        __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
 
-// A warp lists the pairs of the 32 triangles at Morton positions 32 qb + lane
+struct __align__(16) Query {
+    float4 lo, hi;
+    int4 verts;
+};
+
+// A warp lists the pairs of the 32 triangles at curve positions 32 qb + lane
 // with the triangles at later positions (every unordered pair is met once).
 // Blocks are found with the common box, 32 per test, and kept only for the
-// lanes whose own box touches them: 32 neighbours that straddle a jump of the
-// Morton curve have a common box as large as the scene, yet each of them
+// lanes whose own box touches them: 32 neighbours on the curve can lie on
+// different bodies, with a common box much larger than theirs, yet each of them
 // touches a dozen 32-leaf blocks at most.  In a block that is kept, each of
 // those lanes' boxes in turn meets all 32 leaves, one per lane, so the work is
 // the number of (triangle, block) contacts, 3.5 per triangle of a body, however
-// the common box lies (a loop over the leaves that touch the common box took
-// 1620 us for 105k triangles in the warps at such jumps).
+// large the common box is (a loop over the leaves that touch the common box took
+// 1620 us for 105k triangles, in a few warps).
 // emit(src, hits, hit, j): for query lane src, in ascending partner position,
 // the lanes of the ballot `hits` pair it with their triangle j; `on`: the lanes
 // that take part as queries.  Pair rules of broadphase_find_pairs_bvh_kernel
 // (udcf/kernel.py:937-981): static-static never, movable-self only when allowed
-// and sharing no vertex.
+// and sharing no vertex.  s_q: the warp's queries, read back as broadcasts.
 template <class Emit>
-__device__ __forceinline__ void walk_blocks(const XpbdDcd& D, int qb, bool on, Emit emit) {
+__device__ __forceinline__ void walk_blocks(const XpbdDcd& D, int qb, bool on, Query* s_q, Emit emit) {
     const Leaves L(D);
     const int n = D.n_tris, nb = (n + 31) / 32, nk = (n + 1023) / 1024;
     const int lane = threadIdx.x & 31, t = 32 * qb + lane;
     const float4 ulo = L.b32[2 * qb], uhi = L.b32[2 * qb + 1];
     float4 qlo = make_float4(0.f, 0.f, 0.f, 0.f), qhi = qlo;
-    int4 qv = make_int4(-1, -1, -1, 0);
     on = on && t < n;
     if (on) {
-        qlo = L.lo[t];
-        qhi = L.hi[t];
-        qv = L.verts[t];
+        s_q[lane].lo = qlo = L.lo[t];
+        s_q[lane].hi = qhi = L.hi[t];
+        s_q[lane].verts = L.verts[t];
     }
+    __syncwarp();
     for (int k0 = qb >> 5; k0 < nk; k0 += 32) {
         const int k = min(k0 + lane, nk - 1);
         const float4 klo = L.b1k[2 * k], khi = L.b1k[2 * k + 1];
@@ -372,20 +405,19 @@ __device__ __forceinline__ void walk_blocks(const XpbdDcd& D, int qb, bool on, E
                 if (!mq) continue;
                 const int p = 32 * (c0 + cs) + lane, pc = min(p, n - 1);
                 const float4 lo = L.lo[pc], hi = L.hi[pc];
+                const int4 v = L.verts[pc];
                 for (; mq; mq &= mq - 1) {
                     const int src = __ffs(mq) - 1;
-                    const float4 alo = shfl4(qlo, src), ahi = shfl4(qhi, src);
+                    const float4 alo = s_q[src].lo, ahi = s_q[src].hi;
                     bool hit = p < n && p > 32 * qb + src && overlap(alo, ahi, lo, hi);
                     if (!__any_sync(0xffffffffu, hit)) continue;
                     const int g = __float_as_int(hi.w), ag = __float_as_int(ahi.w);
-                    const int a = __shfl_sync(0xffffffffu, qv.x, src), b = __shfl_sync(0xffffffffu, qv.y, src),
-                              d = __shfl_sync(0xffffffffu, qv.z, src);
+                    const int4 q = s_q[src].verts;
                     if (g == 1 && ag == 1) hit = false;
-                    if (hit && g == 0 && ag == 0) {
-                        const int4 v = L.verts[pc];
-                        hit = D.allow_self && !(v.x == a || v.x == b || v.x == d || v.y == a || v.y == b || v.y == d ||
-                                                v.z == a || v.z == b || v.z == d);
-                    }
+                    if (g == 0 && ag == 0)
+                        hit = hit && D.allow_self &&
+                              !(v.x == q.x || v.x == q.y || v.x == q.z || v.y == q.x || v.y == q.y || v.y == q.z ||
+                                v.z == q.x || v.z == q.y || v.z == q.z);
                     const unsigned hits = __ballot_sync(0xffffffffu, hit);
                     if (hits) emit(src, hits, hit, __float_as_int(lo.w));
                 }
@@ -397,12 +429,13 @@ __device__ __forceinline__ void walk_blocks(const XpbdDcd& D, int qb, bool on, E
 // Counting pass: pairs per query (ws_count) and per block of 32 (ws_keys2); a
 // query's first kSlots partners are kept for the fill pass.
 __global__ void __launch_bounds__(128) k_count_pairs(XpbdDcd D) {
+    __shared__ Query s_q[4][32];
     const int qb = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int n = D.n_tris, t = 32 * qb + lane;
     if (32 * qb >= n) return;
     int cnt = 0;
     if (!(*D.status & XPBD_STATUS_BARRIER_TIMEOUT))  // else the sort gave up: no valid order, no pairs
-        walk_blocks(D, qb, true, [&](int src, unsigned hits, bool hit, int j) {
+        walk_blocks(D, qb, true, s_q[threadIdx.x >> 5], [&](int src, unsigned hits, bool hit, int j) {
             const int slot = __shfl_sync(0xffffffffu, cnt, src) + __popc(hits & ((1u << lane) - 1u));
             if (hit && slot < kSlots) D.ws_slots[int64_t(slot) * n + 32 * qb + src] = j;
             if (lane == src) cnt += __popc(hits);
@@ -415,6 +448,7 @@ __global__ void __launch_bounds__(128) k_count_pairs(XpbdDcd D) {
 // Fill pass: pairs as (min, max) triangle id, grouped by query position; only
 // queries with more than kSlots partners walk again.
 __global__ void __launch_bounds__(128) k_fill_pairs(XpbdDcd D) {
+    __shared__ Query s_q[4][32];
     const int qb = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int n = D.n_tris, t = 32 * qb + lane;
     if (32 * qb >= n) return;
@@ -434,7 +468,7 @@ __global__ void __launch_bounds__(128) k_fill_pairs(XpbdDcd D) {
     }
     const bool again = c > kSlots;
     if (__any_sync(0xffffffffu, again))
-        walk_blocks(D, qb, again, [&](int src, unsigned hits, bool hit, int j) {
+        walk_blocks(D, qb, again, s_q[threadIdx.x >> 5], [&](int src, unsigned hits, bool hit, int j) {
             const int k = __shfl_sync(0xffffffffu, out, src) + __popc(hits & ((1u << lane) - 1u));
             const int is = __shfl_sync(0xffffffffu, i, src);
             if (hit && k < D.max_pairs) pairs[k] = make_int2(min(is, j), max(is, j));
