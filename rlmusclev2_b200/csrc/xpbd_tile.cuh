@@ -30,7 +30,7 @@ __device__ __forceinline__ void finish_core(const XpbdParams& prm, int f, float4
         }
     }
     if ((ops & XPBD_APPLY_DIVIDE) && a.w > 1e-9f) {
-        float3 d = make_float3(a.x / a.w, a.y / a.w, a.z / a.w);
+        float3 d = over(f3(a), a.w);
         if (prm.omega != 1.f) d = prm.omega * d;
         p.x += d.x;
         p.y += d.y;
