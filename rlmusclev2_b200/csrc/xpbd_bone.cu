@@ -9,14 +9,16 @@
 // The reference queries a Warp BVH mesh; here the closest-point query is a
 // brute force over the bone faces, staged through shared memory in chunks of
 // kFaceChunk faces (the bone surfaces are small next to the muscle mesh, and
-// the query runs at bind time and on slide frames only).  One thread per
-// muscle vertex.  Barycentric convention of Warp's mesh_eval_position: face
+// the query runs at bind time and on slide frames only).  G threads per muscle
+// vertex share its faces.  Barycentric convention of Warp's mesh_eval_position: face
 // (A, B, C), position(u, v) = u A + v B + (1 - u - v) C; the face frame is the
 // reference's _face_basis (mg/kernel.py:267-285): t1 along position(1,0) -
 // position(0,0) = A - C, n the face normal, t2 = n x t1.  Closest point on a
 // triangle: the Voronoi-region walk of Ericson, Real-Time Collision Detection
 // (2005), sec. 5.1.5; ties between faces keep the lowest face index.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "xpbd_common.cuh"
 #include "xpbd_device.cuh"
@@ -93,8 +95,16 @@ __device__ __forceinline__ FaceFrame face_frame(float3 A, float3 B, float3 C) {
 }
 
 // Closest bone face to p within max_dist (brute force, faces staged in shared
-// memory by the whole CTA).  Every thread of the CTA must call it (it holds
-// __syncthreads); threads past the query count pass active = false.
+// memory by the whole CTA); of equally close faces the lowest index, whatever G
+// is.  G neighbouring lanes hold the same p, take every G-th face each and agree
+// on the result.  Every thread of the CTA must call it (it holds __syncthreads);
+// threads past the query count pass active = false.
+//
+// Bound by the arithmetic of the tests (about 100 instructions each) once the
+// chip is full; with one thread per vertex the 7.6k bound vertices of a body fill
+// 30 CTAs, each thread walking all 1,280 faces: 558 us against 74 us with 32
+// lanes a vertex (random faces; 250 us before on a bone's).
+template <int G>
 __device__ int closest_face(float3 p, bool active, const float4* bone, int nt, const int* tris, float max_dist,
                             float& bu, float& bv, float3 (*s_tri)[3]) {
     int best = -1;
@@ -106,7 +116,7 @@ __device__ int closest_face(float3 p, bool active, const float4* bone, int nt, c
             face_corners(bone, tris, f0 + k, s_tri[k][0], s_tri[k][1], s_tri[k][2]);
         __syncthreads();
         if (active) {
-            for (int k = 0; k < nf; ++k) {
+            for (int k = threadIdx.x & (G - 1); k < nf; k += G) {
                 float u, v;
                 const float d = closest_tri(p, s_tri[k][0], s_tri[k][1], s_tri[k][2], u, v);
                 if (d < bd || (best < 0 && d <= bd)) {
@@ -116,6 +126,18 @@ __device__ int closest_face(float3 p, bool active, const float4* bone, int nt, c
                     bv = v;
                 }
             }
+        }
+    }
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) {
+        const float d = __shfl_xor_sync(0xffffffffu, bd, o), u = __shfl_xor_sync(0xffffffffu, bu, o),
+                    v = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int f = __shfl_xor_sync(0xffffffffu, best, o);
+        if (f >= 0 && (best < 0 || d < bd || (d == bd && f < best))) {
+            bd = d;
+            best = f;
+            bu = u;
+            bv = v;
         }
     }
     return best;
@@ -130,17 +152,18 @@ __device__ __forceinline__ float3 from_local(const FaceFrame& F, float4 l) {
                        F.t1.z * l.x + F.t2.z * l.y + F.n.z * l.z);
 }
 
+template <int G>
 __global__ void __launch_bounds__(kBoneThreads)
     k_bone_bind(int n, const float4* __restrict__ q4, const float4* __restrict__ bone, int nt,
                 const int* __restrict__ tris, float max_dist, int* __restrict__ out_face, float2* __restrict__ out_uv,
                 float4* __restrict__ out_local) {
     __shared__ float3 s_tri[kFaceChunk][3];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const bool active = i < n;
     const float3 p = active ? f3(q4[i]) : make_float3(0.f, 0.f, 0.f);
     float u = 0.f, v = 0.f;
-    const int f = closest_face(p, active, bone, nt, tris, max_dist, u, v, s_tri);
-    if (!active) return;
+    const int f = closest_face<G>(p, active, bone, nt, tris, max_dist, u, v, s_tri);
+    if (!active || threadIdx.x % G) return;
     if (f < 0) {  // nothing within max_dist: the reference writes face 0, zero uv and offset
         out_face[i] = 0;
         out_uv[i] = make_float2(0.f, 0.f);
@@ -156,19 +179,19 @@ __global__ void __launch_bounds__(kBoneThreads)
     out_local[i] = make_float4(l.x, l.y, l.z, 0.f);
 }
 
-template <bool REPROJECT>
+template <bool REPROJECT, int G>
 __global__ void __launch_bounds__(kBoneThreads)
     k_bone_slide_targets(int n, const float4* __restrict__ m4, const int* __restrict__ anchor_face,
                          const float2* __restrict__ anchor_uv, int* __restrict__ bind_face, float2* __restrict__ bind_uv,
                          float4* __restrict__ local4, float slide_range, float max_dist, const float4* __restrict__ bone,
                          int nt, const int* __restrict__ tris, float4* pin_target, float4* attach_target) {
     __shared__ float3 s_tri[REPROJECT ? kFaceChunk : 1][3];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const bool active = i < n && threadIdx.x % G == 0;
     if (REPROJECT) {
-        const float3 p = active ? f3(m4[i]) : make_float3(0.f, 0.f, 0.f);
+        const float3 p = i < n ? f3(m4[i]) : make_float3(0.f, 0.f, 0.f);
         float u = 0.f, v = 0.f;
-        const int f = closest_face(p, active, bone, nt, tris, max_dist, u, v, s_tri);
+        const int f = closest_face<G>(p, i < n, bone, nt, tris, max_dist, u, v, s_tri);
         if (active && f >= 0) {
             float3 A, B, C;
             face_corners(bone, tris, anchor_face[i], A, B, C);
@@ -251,17 +274,18 @@ __global__ void k_m2m_glue(int n, const int* __restrict__ pa, const int* __restr
 // fascia_bind_kernel (fascia/fascia.py:130-157): closest muscle-surface face
 // of each fascia rest vertex, its (u, v) and the signed normal gap
 // (rest - closest point) . n; ok = 0 when nothing lies within max_dist.
+template <int G>
 __global__ void __launch_bounds__(kBoneThreads)
     k_surface_bind(int n, const float4* __restrict__ q4, const float4* __restrict__ surf, int nt,
                    const int* __restrict__ tris, float max_dist, int* __restrict__ out_face, float2* __restrict__ out_uv,
                    float* __restrict__ out_gap, int* __restrict__ out_ok) {
     __shared__ float3 s_tri[kFaceChunk][3];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const bool active = i < n;
     const float3 p = active ? f3(q4[i]) : make_float3(0.f, 0.f, 0.f);
     float u = 0.f, v = 0.f;
-    const int f = closest_face(p, active, surf, nt, tris, max_dist, u, v, s_tri);
-    if (!active) return;
+    const int f = closest_face<G>(p, active, surf, nt, tris, max_dist, u, v, s_tri);
+    if (!active || threadIdx.x % G) return;
     if (f < 0) {
         out_face[i] = 0;
         out_uv[i] = make_float2(0.f, 0.f);
@@ -357,6 +381,22 @@ __global__ void k_fascia_glue(int n, const int* __restrict__ pf, const int* __re
 bool a16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 bool a8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
+unsigned bone_ctas(int n, int G) { return unsigned((int64_t(n) * G + kBoneThreads - 1) / kBoneThreads); }
+
+// Lanes per closest-face query: 32 until 8 lanes fill eight CTAs on each of 148
+// SMs by themselves (37,857 queries), then 8, whose staged faces serve four
+// times the queries.  32 against 8 lanes, 1,280 faces: 74 and 97 us for 7,622
+// queries, 231 and 248 for 30,000, 438 and 434 for 60,000, 2,819 and 2,667 for
+// 400,000; with 300 faces 134 and 114 us for 60,000.  (One lane: 137 to 559 us up
+// to 30,000 queries, 667 and 2,826 us for 400,000.)
+template <class F>
+void with_lanes(int n, F f) {
+    if (bone_ctas(n, 8) >= 8 * 148)
+        f(std::integral_constant<int, 8>{});
+    else
+        f(std::integral_constant<int, 32>{});
+}
+
 }  // namespace
 
 extern "C" {
@@ -370,9 +410,12 @@ int xpbd_bone_bind(int32_t n, const float* query4, int32_t n_bverts, const float
     if (!a16(query4) || !a16(bone4) || !a16(out_local4) || !a8(out_uv))
         return fail(XPBD_ERR_ALIGN, "xpbd_bone_bind: [n][4] arrays 16-byte, uv 8-byte aligned");
     if (n == 0) return XPBD_OK;
-    k_bone_bind<<<(n + kBoneThreads - 1) / kBoneThreads, kBoneThreads, 0, (cudaStream_t)stream>>>(
-        n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(bone4), n_btris, btris, max_dist,
-        out_face, reinterpret_cast<float2*>(out_uv), reinterpret_cast<float4*>(out_local4));
+    with_lanes(n, [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        k_bone_bind<G><<<bone_ctas(n, G), kBoneThreads, 0, (cudaStream_t)stream>>>(
+            n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(bone4), n_btris, btris,
+            max_dist, out_face, reinterpret_cast<float2*>(out_uv), reinterpret_cast<float4*>(out_local4));
+    });
     return cuda_check("xpbd_bone_bind");
 }
 
@@ -388,7 +431,6 @@ int xpbd_bone_slide_targets(int32_t n, const float* muscle4, const int32_t* anch
         !a8(anchor_uv))
         return fail(XPBD_ERR_ALIGN, "xpbd_bone_slide_targets: [n][4] arrays 16-byte, uv 8-byte aligned");
     if (n == 0) return XPBD_OK;
-    const dim3 grid((n + kBoneThreads - 1) / kBoneThreads);
     cudaStream_t s = (cudaStream_t)stream;
 #define XPBD_SLIDE_ARGS                                                                                               \
     n, reinterpret_cast<const float4*>(muscle4), anchor_face, reinterpret_cast<const float2*>(anchor_uv), bind_face, \
@@ -396,9 +438,12 @@ int xpbd_bone_slide_targets(int32_t n, const float* muscle4, const int32_t* anch
         reinterpret_cast<const float4*>(bone4), n_btris, btris, reinterpret_cast<float4*>(pin_target),               \
         reinterpret_cast<float4*>(attach_target)
     if (reproject)
-        k_bone_slide_targets<true><<<grid, kBoneThreads, 0, s>>>(XPBD_SLIDE_ARGS);
+        with_lanes(n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            k_bone_slide_targets<true, G><<<bone_ctas(n, G), kBoneThreads, 0, s>>>(XPBD_SLIDE_ARGS);
+        });
     else
-        k_bone_slide_targets<false><<<grid, kBoneThreads, 0, s>>>(XPBD_SLIDE_ARGS);
+        k_bone_slide_targets<false, 1><<<bone_ctas(n, 1), kBoneThreads, 0, s>>>(XPBD_SLIDE_ARGS);
 #undef XPBD_SLIDE_ARGS
     return cuda_check("xpbd_bone_slide_targets");
 }
@@ -423,9 +468,12 @@ int xpbd_surface_bind(int32_t n, const float* query4, int32_t n_sverts, const fl
     if (!a16(query4) || !a16(surf4) || !a8(out_uv))
         return fail(XPBD_ERR_ALIGN, "xpbd_surface_bind: [n][4] arrays 16-byte, uv 8-byte aligned");
     if (n == 0) return XPBD_OK;
-    k_surface_bind<<<(n + kBoneThreads - 1) / kBoneThreads, kBoneThreads, 0, (cudaStream_t)stream>>>(
-        n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(surf4), n_stris, stris, max_dist,
-        out_face, reinterpret_cast<float2*>(out_uv), out_gap, out_ok);
+    with_lanes(n, [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        k_surface_bind<G><<<bone_ctas(n, G), kBoneThreads, 0, (cudaStream_t)stream>>>(
+            n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(surf4), n_stris, stris,
+            max_dist, out_face, reinterpret_cast<float2*>(out_uv), out_gap, out_ok);
+    });
     return cuda_check("xpbd_surface_bind");
 }
 

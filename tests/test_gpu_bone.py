@@ -197,3 +197,38 @@ def test_multigrid_mesh_from_bone_dir_matches_capsule_pose(tmp_path):
     err = np.abs(sim.positions_np() - sim2.positions_np()).max()
     print(f"bone_dir run vs capsule-pose run: max |diff| {err:.2e} m")
     assert err < 1e-6
+
+
+@pytest.mark.parametrize("n", [1, 9, 33, 6001, 37856, 37857, 151297])
+def test_lanes_per_query_agree(n):
+    """The lanes that share a query's faces depend on the query count (32 below
+    37,857 queries, then 8): both find a closest face.
+
+    Tolerance of the distance: about ten FP32 roundings of coordinates below
+    0.5 m on either side, 2 * 10 * 0.5 * 6e-8 = 6e-7, taken as 1e-6."""
+    lib = capi.load()
+    v, t, _ = _bones()
+    v, t = v[:400], t[(t < 400).all(1)][:389]  # a face count that 8 and 32 do not divide, over one chunk
+    rng = np.random.default_rng(n)
+    q = (v[rng.integers(0, 400, n)] + rng.normal(scale=0.01, size=(n, 3))).astype(np.float32)
+    q[0] = v[t[0, 0]]  # on a vertex: several faces at distance zero, the lowest index wins
+    reach = 0.01
+    face = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    uv = torch.full((n, 2), -7.0, device="cuda")
+    loc = torch.full((n, 4), -7.0, device="cuda")
+    q4, b4, td = _d(_v4(q)), _d(_v4(v)), _d(t)
+    assert lib.xpbd_bone_bind(n, _p(q4), v.shape[0], _p(b4), t.shape[0], _p(td), C.c_float(reach), _p(face), _p(uv),
+                              _p(loc), None) == 0
+    torch.cuda.synchronize()
+    gf, guv, gloc = face.cpu().numpy(), uv.cpu().numpy().astype(np.float64), loc.cpu().numpy()
+    v64 = v.astype(np.float64)
+    pick = rng.permutation(n)[:2000]
+    pick[0] = 0
+    of, ouv, _ = O.bone_bind(q[pick], v, t, 1.0)
+    d_or = np.linalg.norm(q[pick] - _cp(v64, t, of, ouv.astype(np.float64)), axis=1)
+    found = d_or < reach - 1e-6
+    d_gpu = np.linalg.norm(q[pick] - _cp(v64, t, gf[pick], guv[pick]), axis=1)
+    assert np.abs(d_gpu - d_or)[found].max() <= 1e-6
+    none = d_or > reach + 1e-6
+    assert (gf[pick][none] == 0).all() and (guv[pick][none] == 0).all() and (gloc[pick][none] == 0).all()
+    assert gf[0] == np.nonzero((t == t[0, 0]).any(1))[0][0]
