@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes as C
 import logging
+import threading
 
 import numpy as np
 import torch
@@ -148,6 +149,10 @@ class XpbdEngine:
         self._prev4 = self._pos4.clone()
         v4 = np.zeros((nv, 4), np.float32)
         v4[:, 3] = (self._stopped_user != 0)
+        self._vinv_d = T(L.inv.astype(np.int32))
+        self._pos_user = torch.zeros((nv, 3), dtype=f32, device=dev)
+        self._pos_host = torch.zeros((nv, 3), dtype=f32).pin_memory()
+        self._pos_lock = threading.Lock()  # the two buffers above, when threads share an engine
         self._vel4 = T(v4[L.perm])
         self._massd = T(self._mass_user[L.perm])
         self._accum = torch.zeros((nv, 4), dtype=f32, device=dev)
@@ -674,7 +679,22 @@ class XpbdEngine:
         return out
 
     def positions_np(self) -> np.ndarray:
-        return self._to_user(self._pos4)
+        """Positions in the user's vertex order: device gather, one copy into
+        pinned host memory.  (Copied as four columns and put in order on the
+        host, with a pageable copy on another stream, the same call cost 40 to
+        70 us of a 300-vertex frame of 121.)"""
+        with self._pos_lock:
+            # what the caller queued on its own stream comes first
+            self._stream.wait_stream(torch.cuda.current_stream(self.device))
+            capi.check(self._lib.xpbd_gather(self.n_verts, 3, C.c_void_p(self._vinv_d.data_ptr()),
+                                             C.c_void_p(self._pos4.data_ptr()), 4,
+                                             C.c_void_p(self._pos_user.data_ptr()), 3, self._sp))
+            with torch.cuda.stream(self._stream):
+                self._pos_host.copy_(self._pos_user, non_blocking=True)
+            self.synchronize()  # raises on a fatal status bit of the frames before
+            out = torch.empty_like(self._pos_host, pin_memory=False)
+            out.copy_(self._pos_host)  # multi-threaded host copy out of the pinned buffer
+        return out.numpy()
 
     @property
     def pos(self) -> torch.Tensor:

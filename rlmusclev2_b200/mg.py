@@ -353,11 +353,8 @@ class MultiGridSim(MuscleSim):
         r4[:, :3] = self.pos0_np
         self._rest4 = torch.from_numpy(r4[L.perm]).to(dev)
         self._tet_perm_d = torch.from_numpy(L.tet_perm.astype(np.int32)).to(dev)
-        self._vinv_d = torch.from_numpy(L.inv.astype(np.int32)).to(dev)
         self._act_user = torch.zeros(self.NT, dtype=torch.float32, device=dev)
         self._act_host = torch.zeros(self.NT, dtype=torch.float32).pin_memory()
-        self._pos_user = torch.zeros((self.NV, 3), dtype=torch.float32, device=dev)
-        self._pos_host = torch.zeros((self.NV, 3), dtype=torch.float32).pin_memory()
         # One event per pinned staging buffer: a buffer is refilled only after
         # its own previous copy has been consumed, so the activation upload and
         # the target upload of one frame do not wait on each other.
@@ -653,18 +650,6 @@ class MultiGridSim(MuscleSim):
         capi.check(self._lib.xpbd_gather(self.NT, 1, C.c_void_p(self._tet_perm_d.data_ptr()),
                                          C.c_void_p(self._act_user.data_ptr()), 1, C.c_void_p(self._t_act.data_ptr()),
                                          1, self._sp))
-
-    def positions_np(self) -> np.ndarray:
-        """Positions in the user's vertex order: device gather, one D2H copy."""
-        capi.check(self._lib.xpbd_gather(self.NV, 3, C.c_void_p(self._vinv_d.data_ptr()),
-                                         C.c_void_p(self._pos4.data_ptr()), 4, C.c_void_p(self._pos_user.data_ptr()),
-                                         3, self._sp))
-        with torch.cuda.stream(self._stream):
-            self._pos_host.copy_(self._pos_user, non_blocking=True)
-        self.synchronize()  # raises on a fatal status bit of the frames before
-        out = torch.empty((self.NV, 3), dtype=torch.float32)
-        out.copy_(self._pos_host)  # multi-threaded host copy out of the pinned buffer
-        return out.numpy()
 
     # -------------------------------------------------------------- program
     def apply_pintotarget(self) -> None:
