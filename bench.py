@@ -408,7 +408,7 @@ def run_ours(args):
         pass
     hook_persistent = bool(sim._persist_fits and getattr(sim, "persistent_between_hooks", False)
                            and sim.use_persistent)
-    per_iter = (1 if hook_persistent else 2) + (3 if getattr(sim, "dcd", None) is not None else 0)
+    per_iter = (1 if hook_persistent else 2) + (2 if getattr(sim, "dcd", None) is not None else 0)
     fine = len(sim._persist) if persistent else sim.fine_iters * per_iter
     coarse = 0
     if sim.mg is not None:
@@ -419,8 +419,12 @@ def run_ours(args):
         every = max(1, int(sim.dcd.params.bvh_rebuild_every))
         per_sub += sum(sim.dcd.buf.broadphase_launches(True, refit_only=(k % every) != 0)
                        for k in range(sim.nsubsteps)) / sim.nsubsteps
+    # all substeps in one launch per tile range, else a vertex step ends the frame
+    frame_kernel = bool(persistent and sim.persistent_sync == "exchange" and sim._exchange is not None
+                        and not (sim._prm.tile_variant & ~0x53))
+    whole = frame_kernel and sim.mg is None and sim.fascia is None and not sim.n_m2m
     launches_per_frame = 1 + (1 if sim.collision_solvers else 0) + (1 if sim._has_pins else 0) + (
-        1 if sim.mg is not None else 0) + sim.nsubsteps * per_sub + 1
+        1 if sim.mg is not None else 0) + (len(sim._persist) if whole else sim.nsubsteps * per_sub + 1)
     n_iter = sim.nsubsteps * sim.fine_iters
     line = {
         "metric": "ms/frame", "value": round(ms_frame, 4), "unit": "ms/frame", "n_gpus": world, "steps": args.steps,
@@ -438,8 +442,10 @@ def run_ours(args):
         "e2e": {"value": round(ms_e2e, 4), "unit": "ms/frame", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic, "peak_kind": peak_kind,
-                     "kernel": ("k_iterate_persistent (all Jacobi iterations of a substep in one launch; "
-                                "time per iteration, inside a frame)") if persistent else
+                     "kernel": ("k_frame_tiles (all substeps' Jacobi iterations and vertex steps in one launch; "
+                                "time per iteration, inside a frame)") if whole else
+                               (f"{'k_frame_tiles' if frame_kernel else 'k_iterate_persistent'} (all Jacobi iterations "
+                                "of a substep in one launch; time per iteration, inside a frame)") if persistent else
                                ("k_iterate_persistent (one launch per iteration, a hook between iterations)"
                                 if (sim._persist_fits and getattr(sim, "persistent_between_hooks", False)
                                     and sim.collision_solvers_iter and sim.use_persistent)

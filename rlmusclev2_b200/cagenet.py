@@ -26,10 +26,6 @@ OUT_PAD_FWD = 16   # rows of the last layer's weight (n of its GEMM, a multiple 
 OUT_PAD_BWD = 64   # k of the last layer's backward GEMM (a multiple of 64)
 
 
-def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
-
-
 def gemm(lib, stream, a, b, m, n, k, *, lda=None, ldb=None, bias=None, act=0, gelu_grad_of=None, out_pre=None,
          out_f32=None, out_bf16=None, out_bf16_t=None, status=None, n_tile=None, flags=0):
     """C = A B^T (+ epilogue) through xpbd_gemm_bf16; tensors are CUDA, BF16
