@@ -210,11 +210,10 @@ class DcdBuffers:
         self._built = True
 
     def broadphase_launches(self, snapshot_prev: bool = True, refit_only: bool = False) -> int:
-        """Kernels one xpbd_dcd_broadphase call launches: keys and snapshot
-        (neither: no launch), cooperative sort (not when refitting), leaves,
+        """Kernels one xpbd_dcd_broadphase call launches: cooperative sort with
+        keys and snapshot (when refitting only the snapshot, if any), leaves,
         counting pass, scan, fill pass."""
-        rebuild = 0 if refit_only else 1
-        return int(bool(snapshot_prev) or bool(rebuild)) + rebuild + 4
+        return int(bool(snapshot_prev) or not refit_only) + 4
 
     def narrow_respond(self, pos4: torch.Tensor, stream) -> None:
         capi.check(self.lib.xpbd_dcd_narrow_respond(C.byref(self.d), C.c_void_p(pos4.data_ptr()), stream))

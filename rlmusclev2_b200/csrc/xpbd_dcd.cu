@@ -105,14 +105,9 @@ __device__ __forceinline__ uint32_t hilbert24(uint32_t x, uint32_t y, uint32_t z
     return spread10(x ^ t) << 2 | spread10(y ^ t) << 1 | spread10(z ^ t);
 }
 
-// Curve keys into the buffers the first of the sort's three passes reads (8
-// bits per axis: cells of 3.5 mm on the 0.9-m body, about half a triangle; the
-// order only decides how tight the leaf blocks are), and the snapshot of the
-// positions when asked for.
-__global__ void k_tri_keys(XpbdDcd D, const float* __restrict__ pos4, int keys, int snapshot) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (snapshot && i < D.n_verts) reinterpret_cast<float4*>(D.x_prev)[i] = ld4(pos4, i);
-    if (!keys || i >= D.n_tris) return;
+// Curve key of triangle i: 8 bits per axis, cells of 3.5 mm on the 0.9-m body,
+// about half a triangle (the order only decides how tight the leaf blocks are).
+__device__ __forceinline__ uint32_t tri_key(const XpbdDcd& D, const float* __restrict__ pos4, int i) {
     float3 lo, hi;
     tri_box(D, pos4, D.tris[3 * i], D.tris[3 * i + 1], D.tris[3 * i + 2], lo, hi);
     const float q[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
@@ -122,8 +117,13 @@ __global__ void k_tri_keys(XpbdDcd D, const float* __restrict__ pos4, int keys, 
         const float ext = fmaxf(D.box_hi[k] - D.box_lo[k], 1e-30f);
         u[k] = uint32_t(fminf(fmaxf((q[k] - D.box_lo[k]) / ext * 255.f, 0.f), 255.f));
     }
-    D.ws_keys2[i] = hilbert24(u[0], u[1], u[2]);
-    D.ws_vals2[i] = i;
+    return hilbert24(u[0], u[1], u[2]);
+}
+
+// The snapshot of the positions by itself, for a broadphase that does not sort.
+__global__ void k_snapshot(XpbdDcd D, const float* __restrict__ pos4) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < D.n_verts) reinterpret_cast<float4*>(D.x_prev)[i] = ld4(pos4, i);
 }
 
 // ---------------------------------------------------------- radix sort
@@ -193,7 +193,9 @@ __global__ void __launch_bounds__(1024) k_scan_pairs(XpbdDcd D) {
 // first output slot per digit; (C) stable scatter in rounds of kSortThreads
 // keys: warps rank equal digits with __match_any_sync, per-digit prefix over
 // the warps in shared memory; grid barrier before the next pass reads.
-// Odd pass count: the input is in ws_keys2/ws_vals2, the sorted data ends in
+// The first pass forms the keys as it counts them, in ws_keys2/ws_vals2 (as a
+// launch of its own that took 4.8 us for 105k triangles), with the snapshot of the
+// positions when asked for; after three passes the sorted data is in
 // ws_keys/ws_vals.
 __device__ __forceinline__ int add_excl_over_warps(int (*wcnt)[256], int d, int run) {
     for (int ww = 0; ww < kSortThreads / 32; ++ww) {
@@ -204,7 +206,8 @@ __device__ __forceinline__ int add_excl_over_warps(int (*wcnt)[256], int d, int 
     return run;
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, int chunk, uint32_t* sync) {
+__global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, const float* __restrict__ pos4,
+                                                             int snapshot, int chunk, uint32_t* sync) {
     __shared__ int wcnt[kSortThreads / 32][256];
     __shared__ int run[256];
     __shared__ int part[kSortThreads / 256][256];
@@ -218,12 +221,19 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, int chunk
     uint32_t* kd = D.ws_keys;
     int32_t* vd = D.ws_vals;
     GridBarrier bar = grid_barrier_begin(sync);
+    if (snapshot)
+        for (int i = b * kSortThreads + int(threadIdx.x); i < D.n_verts; i += G * kSortThreads)
+            reinterpret_cast<float4*>(D.x_prev)[i] = ld4(pos4, i);
     for (int pass = 0; pass < 3; ++pass) {
         const int shift = 8 * pass;
         // (A) chunk histogram
         if (threadIdx.x < 256) run[threadIdx.x] = 0;
         __syncthreads();
         for (int i = beg + int(threadIdx.x); i < end; i += kSortThreads) {
+            if (pass == 0) {  // the chunk's keys; (C) reads them in the same CTA
+                ks[i] = tri_key(D, pos4, i);
+                vs[i] = i;
+            }
             const int dig = int((ks[i] >> shift) & 255u);
             const unsigned peers = __match_any_sync(__activemask(), dig);
             if ((peers & ((1u << lane) - 1u)) == 0) atomicAdd(&run[dig], __popc(peers));
@@ -724,7 +734,7 @@ __global__ void k_dcd_apply(XpbdDcd D, float* pos4) {
 // Sort CTAs: one per kSortThreads keys, at most the co-resident count.
 int64_t hist_words(int n) { return int64_t(256) * ((n + kSortThreads - 1) / kSortThreads); }
 
-int launch_sort(const XpbdDcd* D, uint32_t* sync, cudaStream_t s) {
+int launch_sort(const XpbdDcd* D, const float* pos4, int snapshot, uint32_t* sync, cudaStream_t s) {
     static int slots[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cuda_check("xpbd_dcd_broadphase: device");
@@ -749,7 +759,7 @@ int launch_sort(const XpbdDcd* D, uint32_t* sync, cudaStream_t s) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_sort_coop, *D, chunk, sync) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, k_sort_coop, *D, pos4, snapshot, chunk, sync) != cudaSuccess)
         return cuda_check("xpbd_dcd_broadphase: sort launch");
     return XPBD_OK;
 }
@@ -789,9 +799,11 @@ int xpbd_dcd_broadphase(const XpbdDcd* D, const float* pos4, int32_t snapshot_pr
     if (!pos4 || !aligned16(pos4)) return fail(XPBD_ERR_ARG, "xpbd_dcd_broadphase: pos4");
     cudaStream_t s = (cudaStream_t)stream;
     const int n = D->n_tris;
-    const int rows = std::max(D->refit_only ? 0 : n, snapshot_prev ? D->n_verts : 0);
-    if (rows > 0) k_tri_keys<<<(rows + 255) / 256, 256, 0, s>>>(*D, pos4, D->refit_only ? 0 : 1, snapshot_prev);
-    if (!D->refit_only && (rc = launch_sort(D, reinterpret_cast<uint32_t*>(D->ws_hist + hist_words(n)), s))) return rc;
+    if (D->refit_only) {
+        if (snapshot_prev) k_snapshot<<<(D->n_verts + 255) / 256, 256, 0, s>>>(*D, pos4);
+    } else if ((rc = launch_sort(D, pos4, snapshot_prev, reinterpret_cast<uint32_t*>(D->ws_hist + hist_words(n)), s))) {
+        return rc;
+    }
     k_leaves<<<(n + 1023) / 1024, 1024, 0, s>>>(*D, pos4);
     k_count_pairs<<<(n + 127) / 128, 128, 0, s>>>(*D);
     k_scan_pairs<<<1, 1024, 0, s>>>(*D);
