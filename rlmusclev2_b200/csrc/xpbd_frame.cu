@@ -19,11 +19,10 @@
 // tile waits for tiles it shares nothing with.  The barrier alone took 2.2 us of
 // a 5.5-us iteration (17.6k tets, clock64 stamps) however small the mesh; with
 // the mailboxes and one pass over the vertices per iteration that iteration
-// takes 3.8 us, and 3.2 us with the divisions of the finish and the fibre and
-// volume terms kept per material or done once.  Frames of 200 iterations,
-// device time against a launch per substep boundary and tet pass: 68k tets
-// 1,288 -> 914 us, 222k tets 2.06 -> 1.73 ms; a 12,288-tet box of 10 iterations
-// 113 -> 59 us.
+// takes 3.8 us, and 3.6 us with the constants of the attachments and the fibre
+// and volume terms kept per material.  Frames of 200 iterations, device time
+// against a launch per substep boundary and tet pass: 68k tets 1,288 -> 943 us,
+// 222k tets 2.06 -> 1.72 ms; a 12,288-tet box of 10 iterations 113 -> 66 us.
 //
 // Two slots suffice: a tile stores iteration k + 2 only after it has read every
 // neighbour's k + 1, which that neighbour sent after it had read k.  The
