@@ -481,7 +481,7 @@ typedef struct XpbdDcd {
     float max_push;           /* > 0: clamp contact depth (UdcfParams.max_push) */
     float box_lo[3], box_hi[3]; /* Hilbert-curve quantisation box (centres outside are clamped) */
     int32_t* pairs;           /* [max_pairs][2] (i, j > i), deterministic order; 16-byte aligned */
-    int32_t* n_pairs;         /* [1] candidate pairs found (may exceed max_pairs) */
+    int32_t* n_pairs;         /* [1] candidate pairs found (may exceed max_pairs; at most INT32_MAX) */
     int32_t* n_contacts;      /* [1] contacts found (may exceed max_contacts) */
     int32_t* c_ids;           /* [max_contacts][8]: cur tri verts, pair index, closest tri verts, 0 */
     float* c_data;            /* [max_contacts][12]: n.xyz, C, b1.xyz, C1, b2.xyz, C2 */

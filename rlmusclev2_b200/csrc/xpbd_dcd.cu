@@ -126,51 +126,57 @@ __global__ void k_snapshot(XpbdDcd D, const float* __restrict__ pos4) {
     if (i < D.n_verts) reinterpret_cast<float4*>(D.x_prev)[i] = ld4(pos4, i);
 }
 
+__device__ __forceinline__ uint32_t saturate(unsigned long long v) { return uint32_t(min(v, 0x7fffffffull)); }
+
 // ---------------------------------------------------------- radix sort
-__device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int* block_total) {
+template <class T>
+__device__ __forceinline__ T block_excl_scan(T v, T* warp_sums, T* block_total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
+    T x = v;
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        const T y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
     if (lane == 31) warp_sums[w] = x;
     __syncthreads();
     if (w == 0) {
-        int t = lane < int(blockDim.x >> 5) ? warp_sums[lane] : 0;
+        T t = lane < int(blockDim.x >> 5) ? warp_sums[lane] : T(0);
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, t, o);
+            const T y = __shfl_up_sync(0xffffffffu, t, o);
             if (lane >= o) t += y;
         }
         warp_sums[lane] = t;
     }
     __syncthreads();
-    const int incl = x + (w > 0 ? warp_sums[w - 1] : 0);
+    const T incl = x + (w > 0 ? warp_sums[w - 1] : T(0));
     if (block_total && threadIdx.x == blockDim.x - 1) *block_total = incl;
     return incl - v;
 }
 
 // One CTA: the pair counts of the query blocks become offsets (a 32nd of the
-// triangles: 3,287 values at 105k), their sum the pair count.
+// triangles: 3,287 values at 105k), their sum the pair count.  n triangles can
+// have n (n - 1) / 2 pairs, beyond 32 bits from 65,537 triangles in one place on:
+// the sums are 64 bits wide, and what is stored stops at INT32_MAX, which no
+// list is longer than.
 __global__ void __launch_bounds__(1024) k_scan_pairs(XpbdDcd D) {
-    __shared__ int warp_sums[32];
-    __shared__ int carry, round_total;
-    int* a = reinterpret_cast<int*>(D.ws_keys2);
+    __shared__ unsigned long long warp_sums[32], carry, round_total;
+    uint32_t* a = D.ws_keys2;
     const int nb = (D.n_tris + 31) / 32;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int b0 = 0; b0 < nb; b0 += 1024 * kScanItems) {
         const int base = b0 + int(threadIdx.x) * kScanItems;
-        int v[kScanItems], run = 0;
+        uint32_t v[kScanItems];
+        unsigned long long run = 0;
 #pragma unroll
         for (int q = 0; q < kScanItems; ++q) {
             v[q] = base + q < nb ? a[base + q] : 0;
             run += v[q];
         }
-        int off = block_excl_scan(run, warp_sums, &round_total) + carry;
+        unsigned long long off = block_excl_scan(run, warp_sums, &round_total) + carry;
 #pragma unroll
         for (int q = 0; q < kScanItems; ++q) {
-            if (base + q < nb) a[base + q] = off;
+            if (base + q < nb) a[base + q] = saturate(off);
             off += v[q];
         }
         __syncthreads();
@@ -178,9 +184,9 @@ __global__ void __launch_bounds__(1024) k_scan_pairs(XpbdDcd D) {
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        *D.ws_total = carry;
-        *D.n_pairs = carry;
-        if (carry > D.max_pairs) atomicOr(D.status, XPBD_STATUS_PAIR_OVERFLOW);
+        *D.ws_total = int(saturate(carry));
+        *D.n_pairs = int(saturate(carry));
+        if (carry > uint32_t(D.max_pairs)) atomicOr(D.status, XPBD_STATUS_PAIR_OVERFLOW);
         *D.n_contacts = 0;
     }
 }
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_coop(XpbdDcd D, const flo
                     p_all += wcnt[k][d];
                 }
             }
-            const int base = block_excl_scan(q == 0 ? t_all : 0, warp_sums, nullptr);
+            const int base = block_excl_scan<int>(q == 0 ? t_all : 0, warp_sums, nullptr);
             if (q == 0) run[d] = base + p_all;
             __syncthreads();
         }
@@ -355,8 +361,10 @@ __global__ void __launch_bounds__(1024) k_leaves(XpbdDcd D, const float* __restr
 }
 
 // ------------------------------------------------------------ traversal
+// False for a NaN box (a triangle with an axis on which no corner is a number):
+// it pairs with nothing, where the negated test made it a neighbour of all.
 __device__ __forceinline__ bool overlap(float4 alo, float4 ahi, float4 blo, float4 bhi) {
-    return !(alo.x > bhi.x || blo.x > ahi.x || alo.y > bhi.y || blo.y > ahi.y || alo.z > bhi.z || blo.z > ahi.z);
+    return alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z;
 }
 
 __device__ __forceinline__ float4 shfl4(float4 v, int src) {
@@ -451,8 +459,9 @@ __global__ void __launch_bounds__(128) k_count_pairs(XpbdDcd D) {
             if (lane == src) cnt += __popc(hits);
         });
     if (t < n) D.ws_count[t] = cnt;
-    const int total = __reduce_add_sync(0xffffffffu, cnt);
-    if (lane == 0) reinterpret_cast<int*>(D.ws_keys2)[qb] = total;
+    unsigned long long total = unsigned(cnt);
+    for (int o = 16; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    if (lane == 0) D.ws_keys2[qb] = uint32_t(min(total, 0xffffffffull));
 }
 
 // Fill pass: pairs as (min, max) triangle id, grouped by query position; only
@@ -462,26 +471,29 @@ __global__ void __launch_bounds__(128) k_fill_pairs(XpbdDcd D) {
     const int qb = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int n = D.n_tris, t = 32 * qb + lane;
     if (32 * qb >= n) return;
-    const int c = t < n ? D.ws_count[t] : 0;
-    if (!__any_sync(0xffffffffu, c != 0)) return;
-    int out = c;
+    // unsigned, and stopped at INT32_MAX before each sum: no index wraps into the list
+    const uint32_t base = D.ws_keys2[qb], cap = uint32_t(D.max_pairs);
+    const uint32_t c = t < n && base < cap ? uint32_t(D.ws_count[t]) : 0u;
+    if (!__any_sync(0xffffffffu, c != 0u)) return;
+    uint32_t out = c;
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, out, o);
-        if (lane >= o) out += y;
+        const uint32_t y = __shfl_up_sync(0xffffffffu, out, o);
+        if (lane >= o) out = min(out + y, 0x7fffffffu);
     }
-    out += reinterpret_cast<const int*>(D.ws_keys2)[qb] - c;
+    out = __shfl_up_sync(0xffffffffu, out, 1);
+    out = lane == 0 ? base : min(out + base, 0x7fffffffu);
     const int i = c ? D.ws_vals[t] : 0;
     int2* pairs = reinterpret_cast<int2*>(D.pairs);
-    for (int k = 0; k < c && c <= kSlots; ++k) {
+    for (uint32_t k = 0; k < c && c <= kSlots; ++k) {
         const int j = D.ws_slots[int64_t(k) * n + t];
-        if (out + k < D.max_pairs) pairs[out + k] = make_int2(min(i, j), max(i, j));
+        if (out + k < cap) pairs[out + k] = make_int2(min(i, j), max(i, j));
     }
-    const bool again = c > kSlots;
+    const bool again = c > kSlots && out < cap;
     if (__any_sync(0xffffffffu, again))
         walk_blocks(D, qb, again, s_q[threadIdx.x >> 5], [&](int src, unsigned hits, bool hit, int j) {
-            const int k = __shfl_sync(0xffffffffu, out, src) + __popc(hits & ((1u << lane) - 1u));
+            const uint32_t k = __shfl_sync(0xffffffffu, out, src) + __popc(hits & ((1u << lane) - 1u));
             const int is = __shfl_sync(0xffffffffu, i, src);
-            if (hit && k < D.max_pairs) pairs[k] = make_int2(min(is, j), max(is, j));
+            if (hit && k < cap) pairs[k] = make_int2(min(is, j), max(is, j));
             if (lane == src) out += __popc(hits);
         });
 }
@@ -541,7 +553,8 @@ __device__ __forceinline__ void respond(const XpbdDcd& D, const float* pos4, int
 // One pair; a contact is listed and responded to at once (the responses go to
 // the accumulator, no position moves before k_dcd_apply).
 __device__ __forceinline__ void narrow_pair(const XpbdDcd& D, const float* __restrict__ pos4, int k) {
-    const int ta = D.pairs[2 * k], tb = D.pairs[2 * k + 1];
+    const int2 pair = reinterpret_cast<const int2*>(D.pairs)[k];
+    const int ta = pair.x, tb = pair.y;
     const float3 q00 = f3(ld4(pos4, D.tris[3 * ta])), q01 = f3(ld4(pos4, D.tris[3 * ta + 1])),
                  q02 = f3(ld4(pos4, D.tris[3 * ta + 2]));
     const float3 q10 = f3(ld4(pos4, D.tris[3 * tb])), q11 = f3(ld4(pos4, D.tris[3 * tb + 1])),
@@ -663,8 +676,9 @@ __device__ __forceinline__ void narrow_pair(const XpbdDcd& D, const float* __res
 // The pair count is known on the device only: a grid that fills the GPU strides
 // over it (a thread per possible pair was 16,384 CTAs, 17 us to find 31k pairs).
 __global__ void __launch_bounds__(256) k_narrow(XpbdDcd D, const float* __restrict__ pos4) {
-    const int np = min(*D.n_pairs, D.max_pairs);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) narrow_pair(D, pos4, k);
+    const uint32_t np = uint32_t(min(*D.n_pairs, D.max_pairs));
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x)
+        narrow_pair(D, pos4, int(k));
 }
 
 // respond_kernel (udcf/kernel.py:713-806)

@@ -170,3 +170,64 @@ def test_pairs_at_block_edges(n):
     got = a["pairs"][np.lexsort((a["pairs"][:, 1], a["pairs"][:, 0]))]
     np.testing.assert_array_equal(got, ref)
     np.testing.assert_array_equal(a["pairs"], b["pairs"])
+
+
+@pytest.mark.parametrize("n", [70_000, 100_000])
+def test_pair_count_beyond_32_bits_stops_at_the_list(n):
+    """n disjoint triangles in one place have n (n - 1) / 2 pairs: 2.4e9 and
+    5.0e9, beyond 31 and 32 bits.  The count stops at INT32_MAX, the list is
+    full of the first query's pairs, and nothing is written behind it."""
+    import ctypes
+    lib = capi.load()
+    tri = np.array([[0.0, 0.0, 0.0], [0.01, 0.0, 0.0], [0.0, 0.01, 0.0]], np.float32)
+    p4 = np.ones((3 * n, 4), np.float32)
+    p4[:, :3] = np.tile(tri, (n, 1))
+    tris = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    prm = UdcfParams(allow_self=True, max_pairs=8192, max_contacts=1 << 10)
+    s = torch.cuda.Stream()
+    buf = DcdBuffers(lib, torch.device("cuda:0"), tris, 3 * n, prm, p4[:, :3].min(0) - 0.1, p4[:, :3].max(0) + 0.1)
+    cap = 1000
+    buf.d.max_pairs = cap
+    buf.t["pairs"].fill_(-7)
+    torch.cuda.synchronize()
+    p = torch.from_numpy(p4).cuda()
+    torch.cuda.synchronize()
+    buf.broadphase(p, True, ctypes.c_void_p(s.cuda_stream))
+    s.synchronize()
+    c = buf.counters()
+    assert c["n_pairs"] == 2**31 - 1
+    assert c["status"] == capi.STATUS_PAIR_OVERFLOW
+    pairs = buf.t["pairs"].cpu().numpy()
+    np.testing.assert_array_equal(pairs[:cap], np.stack([np.zeros(cap), np.arange(1, cap + 1)], 1))  # one cell: id order
+    assert (pairs[cap:] == -7).all()
+
+
+def test_triangles_that_are_not_numbers_have_no_pairs():
+    """Triangles with NaN corners pair with nothing; all other pairs are the oracle's."""
+    tris, p4 = _scene_surface()
+    rng = np.random.default_rng(1)
+    bad_tri = rng.choice(tris.shape[0], 40, replace=False)
+    bad_v = np.unique(tris[bad_tri])
+    q4 = p4.copy()
+    q4[bad_v, :3] = np.nan
+    gone = np.isnan(q4[tris, :3]).all(1).any(1)  # an axis without a number; else the box of the other corners
+    keep = np.flatnonzero(~gone)
+    prm = UdcfParams(allow_self=True, thickness=0.0005, max_pairs=1 << 21, max_contacts=1 << 18)
+    lib, s = capi.load(), torch.cuda.Stream()
+    sp = __import__("ctypes").c_void_p(s.cuda_stream)
+    buf = DcdBuffers(lib, torch.device("cuda:0"), tris, p4.shape[0], prm, p4[:, :3].min(0) - 0.01,
+                     p4[:, :3].max(0) + 0.01)
+    p = torch.from_numpy(q4).cuda()
+    torch.cuda.synchronize()
+    buf.broadphase(p, True, sp)
+    s.synchronize()
+    c = buf.counters()
+    got = buf.t["pairs"][:c["n_pairs"]].cpu().numpy()
+    got = got[np.lexsort((got[:, 1], got[:, 0]))]
+    assert c["status"] == 0 and not np.isin(got, np.flatnonzero(gone)).any()
+    # the kept triangles that lost no corner: the same pairs among themselves
+    whole = np.flatnonzero(~np.isnan(q4[tris, :3]).any((1, 2)))
+    ref, _ = O.dcd_pairs(tris, p4, thickness=prm.thickness, allow_self=True)
+    both = lambda a: a[np.isin(a, whole).all(1)]  # noqa: E731
+    np.testing.assert_array_equal(both(got), both(ref))
+    assert len(keep) < tris.shape[0] and len(both(ref)) > 1000
