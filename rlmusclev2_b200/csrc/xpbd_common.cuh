@@ -29,6 +29,23 @@ inline int cuda_check(const char* where) {
     }
     return XPBD_OK;
 }
+// Lets a kernel have `smem` bytes of dynamic shared memory; false where a block
+// cannot.  The limit is a property of the kernel, not of the launch: it is set to
+// the most the device gives, never to one launch's size, so that another thread's
+// launch of the same kernel with smaller tiles cannot lower it in between.
+template <class K>
+bool allow_smem(K kern, size_t smem) {
+    if (smem <= kSmemOptIn) return true;
+    int dev = 0, most = 0;
+    cudaFuncAttributes a;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&a, kern) != cudaSuccess)
+        return false;
+    most -= int(a.sharedSizeBytes);
+    return smem <= size_t(most) &&
+           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+}
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace xpbd

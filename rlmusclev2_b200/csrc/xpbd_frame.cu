@@ -328,11 +328,10 @@ int launch_v(const Launch& L) {
     const size_t smem = (FIXED ? size_t(kFixV) * fix + size_t(L.T->max_tile_verts) * (kSmemPerVert - fix)
                                : size_t(L.T->max_tile_verts) * kSmemPerVert) +
                         size_t(L.max_items) * sizeof(int2);
-    if (smem > kSmemOptIn &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-        if (!L.slots) return cuda_check("xpbd_frame_persistent: smem attribute");
+    if (!allow_smem(kern, smem)) {
         cudaGetLastError();
-        *L.slots = 0;  // the tile does not fit an SM
+        if (!L.slots) return fail(XPBD_ERR_LIMIT, "xpbd_frame_persistent: a tile's vertices and items exceed an SM");
+        *L.slots = 0;
         return XPBD_OK;
     }
     int dev = 0, n_sm = 0, per_sm = 0;

@@ -194,9 +194,10 @@ int launch_v(const XpbdParams* prm, const XpbdTiles* T, const XpbdVerts* V, cons
     const size_t smem = FIXED ? size_t(kFixV) * (4 * sizeof(int) + sizeof(float4)) +
                                     size_t(T->max_tile_verts) * (3 * sizeof(float4) + 2 * sizeof(int))
                               : size_t(T->max_tile_verts) * kSmemPerVert;
-    if (smem > kSmemOptIn &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-        return cuda_check("xpbd_iterate_persistent: smem attribute");
+    if (!allow_smem(kern, smem)) {
+        if (const int rc = cuda_check("xpbd_iterate_persistent: smem attribute")) return rc;
+        return fail(XPBD_ERR_CUDA, "xpbd_iterate_persistent: a tile's vertices exceed an SM's shared memory");
+    }
     int dev = 0, n_sm = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||

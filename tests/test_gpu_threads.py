@@ -1,0 +1,58 @@
+"""Several engines at once: one thread and one stream each."""
+import threading
+
+import numpy as np
+import pytest
+
+from rlmusclev2_b200 import MuscleSim
+from rlmusclev2_b200.meshgen import box_muscle
+from tests.test_gpu_frame import BOX
+
+pytestmark = pytest.mark.gpu
+
+
+def _in_threads(jobs):
+    """Run the jobs at the same time; the first exception of any is raised."""
+    errors, gate = [], threading.Barrier(len(jobs))
+
+    def go(job):
+        try:
+            gate.wait(30)
+            job()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    ts = [threading.Thread(target=go, args=(j,)) for j in jobs]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    if errors:
+        raise errors[0]
+
+
+def _box(tile_tets=None, dims=(8, 8, 32)):
+    m = box_muscle(*dims)
+    return MuscleSim.from_procedural(m.verts, m.tets, m.fiber_per_tet, stopped=m.stopped, tile_tets=tile_tets, **BOX)
+
+
+@pytest.mark.parametrize("sync", ["exchange", "grid"])
+def test_threads_with_different_shared_memory(sync):
+    """Two engines whose tiles need 60 and 66 KB of shared memory launch the
+    same kernel instance from two threads: neither lowers the other's limit."""
+    sims = [_box(2048), _box(3000)]
+    for s in sims:
+        s.use_graphs = False
+        s.persistent_sync = sync
+        s.synchronize()
+
+    def run(s):
+        def job():
+            for _ in range(3000):
+                s._fused_iterations(1)
+        return job
+
+    _in_threads([run(s) for s in sims])
+    for s in sims:
+        assert s.persistent_status() == 0
+        assert np.isfinite(s.positions_np()).all()
