@@ -476,15 +476,17 @@ extern "C" int xpbd_mlp_forward(const XpbdMlp* p, int32_t train, xpbd_stream_t s
         if (!aligned16(p->z[l]) || !aligned16(p->ht[l]))
             return fail(XPBD_ERR_ALIGN, "xpbd_mlp_forward: z and ht must be 16-byte aligned");
     }
+    // before the maps: in a thread's first call it makes the device's context
+    // current, without which the driver encodes none
+    auto kern = train ? k_mlp_chain<TRAIN> : k_mlp_chain<INFER>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) != cudaSuccess)
+        return cuda_check("xpbd_mlp_forward: smem attribute");
     ChainMaps maps;
     bool enc = encode_sw128(&maps.x, p->x, p->m_pad, 64, 64, 16);
     for (int l = 0; l < 5 && enc; ++l)
         enc = encode_sw128(&maps.w[l], p->w[l], l == 4 ? 16 : kHid, l == 0 ? 64 : kHid, l == 0 ? 64 : kHid,
                            l == 4 ? 16 : kHid);
     if (!enc) return fail(XPBD_ERR_CUDA, "xpbd_mlp_forward: tensor maps");
-    auto kern = train ? k_mlp_chain<TRAIN> : k_mlp_chain<INFER>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) != cudaSuccess)
-        return cuda_check("xpbd_mlp_forward: smem attribute");
     kern<<<p->m_pad / kRows, kChainThreads, kChainSmem, (cudaStream_t)stream>>>(*p, maps);
     return cuda_check("xpbd_mlp_forward");
 }
@@ -502,6 +504,11 @@ extern "C" int xpbd_mlp_backward(const XpbdMlp* p, xpbd_stream_t stream) {
             (l < 4 && (!aligned16(p->z[l]) || !aligned16(p->ht[l]) || !aligned16(p->dzt[l]))))
             return fail(XPBD_ERR_ALIGN, "xpbd_mlp_backward: 16-byte alignment");
     }
+    // first, as in xpbd_mlp_forward
+    if (cudaFuncSetAttribute(k_mlp_chain<BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGradSmem)) != cudaSuccess)
+        return cuda_check("xpbd_mlp_backward: smem attribute");
     ChainMaps cm = {};
     bool enc = true;
     for (int l = 0; l < 4 && enc; ++l) {  // wt[4] (k 64), wt[3], wt[2], wt[1]
@@ -515,10 +522,6 @@ extern "C" int xpbd_mlp_backward(const XpbdMlp* p, xpbd_stream_t stream) {
         enc = enc && encode_sw128(&gm.b[l], l == 0 ? p->xt : p->ht[l - 1], l == 0 ? 64 : kHid, M, M, kGradN);
     }
     if (!enc) return fail(XPBD_ERR_CUDA, "xpbd_mlp_backward: tensor maps");
-    if (cudaFuncSetAttribute(k_mlp_chain<BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChainSmem)) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGradSmem)) != cudaSuccess)
-        return cuda_check("xpbd_mlp_backward: smem attribute");
     k_mlp_chain<BACK><<<M / kRows, kChainThreads, kChainSmem, (cudaStream_t)stream>>>(*p, cm);
     k_mlp_wgrad<<<kGradTiles + kSumCtas, kGradThreads, kGradSmem, (cudaStream_t)stream>>>(*p, gm);
     return cuda_check("xpbd_mlp_backward");

@@ -3,8 +3,10 @@ import threading
 
 import numpy as np
 import pytest
+import torch
 
 from rlmusclev2_b200 import MuscleSim
+from rlmusclev2_b200.cagenet import CageMLP
 from rlmusclev2_b200.meshgen import box_muscle
 from tests.test_gpu_frame import BOX
 
@@ -56,3 +58,17 @@ def test_threads_with_different_shared_memory(sync):
     for s in sims:
         assert s.persistent_status() == 0
         assert np.isfinite(s.positions_np()).all()
+
+
+def test_network_in_a_fresh_thread():
+    """A thread whose first CUDA call is the network's: the launches bring the
+    device's context along, for the tensor maps too."""
+    net = CageMLP("cuda:0", 200, stream=torch.cuda.Stream())
+    target = torch.ones((200, 3), device="cuda")
+    torch.cuda.synchronize()
+    _in_threads([lambda: net.forward(200, train=False)])
+    _in_threads([lambda: net.forward(200)])
+    _in_threads([lambda: net.backward(200, target)])
+    torch.cuda.synchronize()
+    assert int(net.status.item()) == 0
+    assert float(net.loss.item()) == 600.0  # features and biases are zero, so are the outputs
