@@ -152,13 +152,19 @@ __device__ __forceinline__ float3 from_local(const FaceFrame& F, float4 l) {
                        F.t1.z * l.x + F.t2.z * l.y + F.n.z * l.z);
 }
 
+// The query of this thread (the threads of a launch pass 32 bits before its queries do).
+template <int G>
+__device__ __forceinline__ int query_index() {
+    return int(blockIdx.x * unsigned(kBoneThreads / G) + threadIdx.x / G);
+}
+
 template <int G>
 __global__ void __launch_bounds__(kBoneThreads)
     k_bone_bind(int n, const float4* __restrict__ q4, const float4* __restrict__ bone, int nt,
                 const int* __restrict__ tris, float max_dist, int* __restrict__ out_face, float2* __restrict__ out_uv,
                 float4* __restrict__ out_local) {
     __shared__ float3 s_tri[kFaceChunk][3];
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int i = query_index<G>();
     const bool active = i < n;
     const float3 p = active ? f3(q4[i]) : make_float3(0.f, 0.f, 0.f);
     float u = 0.f, v = 0.f;
@@ -186,7 +192,7 @@ __global__ void __launch_bounds__(kBoneThreads)
                          float4* __restrict__ local4, float slide_range, float max_dist, const float4* __restrict__ bone,
                          int nt, const int* __restrict__ tris, float4* pin_target, float4* attach_target) {
     __shared__ float3 s_tri[REPROJECT ? kFaceChunk : 1][3];
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int i = query_index<G>();
     const bool active = i < n && threadIdx.x % G == 0;
     if (REPROJECT) {
         const float3 p = i < n ? f3(m4[i]) : make_float3(0.f, 0.f, 0.f);
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(kBoneThreads)
                    const int* __restrict__ tris, float max_dist, int* __restrict__ out_face, float2* __restrict__ out_uv,
                    float* __restrict__ out_gap, int* __restrict__ out_ok) {
     __shared__ float3 s_tri[kFaceChunk][3];
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int i = query_index<G>();
     const bool active = i < n;
     const float3 p = active ? f3(q4[i]) : make_float3(0.f, 0.f, 0.f);
     float u = 0.f, v = 0.f;

@@ -232,3 +232,26 @@ def test_lanes_per_query_agree(n):
     none = d_or > reach + 1e-6
     assert (gf[pick][none] == 0).all() and (guv[pick][none] == 0).all() and (gloc[pick][none] == 0).all()
     assert gf[0] == np.nonzero((t == t[0, 0]).any(1))[0][0]
+
+
+def test_more_queries_than_32_bit_threads():
+    """2^29 + 64 queries of one face: eight lanes each are more threads than 32
+    bits count, and every query is answered all the same (24 GB of buffers)."""
+    lib = capi.load()
+    n = 2**29 + 64
+    if torch.cuda.get_device_properties(0).total_memory < 40e9:
+        pytest.skip("needs 24 GB")
+    q4 = torch.zeros((n, 4), device="cuda")
+    q4[:, 2] = 0.5
+    b4, td = _d(_v4(np.float32([[-1, -1, 0], [3, -1, 0], [-1, 3, 0]]))), _d(np.int32([[0, 1, 2]]))
+    face = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    uv = torch.full((n, 2), -7.0, device="cuda")
+    loc = torch.full((n, 4), -7.0, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.xpbd_bone_bind(n, _p(q4), 3, _p(b4), 1, _p(td), C.c_float(1.0), _p(face), _p(uv), _p(loc), None) == 0
+    torch.cuda.synchronize()
+    assert int((face != 0).sum()) == 0
+    for k in (0, 2**28, 2**29 - 1, 2**29, n - 1):
+        assert abs(float(loc[k, 2]) - 0.5) < 1e-6 and float(uv[k, 0]) > 0.0
+    del q4, face, uv, loc
+    torch.cuda.empty_cache()
