@@ -389,15 +389,20 @@ bool a8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
 unsigned bone_ctas(int n, int G) { return unsigned((int64_t(n) * G + kBoneThreads - 1) / kBoneThreads); }
 
-// Lanes per closest-face query: 32 until 8 lanes fill eight CTAs on each of 148
-// SMs by themselves (37,857 queries), then 8, whose staged faces serve four
-// times the queries.  32 against 8 lanes, 1,280 faces: 74 and 97 us for 7,622
-// queries, 231 and 248 for 30,000, 438 and 434 for 60,000, 2,819 and 2,667 for
-// 400,000; with 300 faces 134 and 114 us for 60,000.  (One lane: 137 to 559 us up
-// to 30,000 queries, 667 and 2,826 us for 400,000.)
+// Lanes per closest-face query: one where the faces number less than a thousandth
+// of the queries (a lane's share of a short list does not pay for its thread and
+// the agreement); else 32 until 8 lanes fill eight CTAs on each of 148 SMs by
+// themselves (37,857 queries), then 8, whose staged faces serve four times the
+// queries.  us with 1, 8 and 32 lanes, 12 faces: 14.6, 10.6 and 13.1 for 10,000
+// queries, 14.9, 14.5 and 23.0 for 30,000, 38, 66 and 183 for 400,000; 100 faces:
+// 53, 31 and 37 for 30,000, 97, 100 and 146 for 150,000, 234, 246 and 368 for
+// 400,000; 1,280 faces: 564, 251 and 231 for 30,000, 875, 559 and 576 for 80,000,
+// 2,834, 2,664 and 2,799 for 400,000.
 template <class F>
-void with_lanes(int n, F f) {
-    if (bone_ctas(n, 8) >= 8 * 148)
+void with_lanes(int n, int n_faces, F f) {
+    if (n_faces < n / 1000)
+        f(std::integral_constant<int, 1>{});
+    else if (bone_ctas(n, 8) >= 8 * 148)
         f(std::integral_constant<int, 8>{});
     else
         f(std::integral_constant<int, 32>{});
@@ -416,7 +421,7 @@ int xpbd_bone_bind(int32_t n, const float* query4, int32_t n_bverts, const float
     if (!a16(query4) || !a16(bone4) || !a16(out_local4) || !a8(out_uv))
         return fail(XPBD_ERR_ALIGN, "xpbd_bone_bind: [n][4] arrays 16-byte, uv 8-byte aligned");
     if (n == 0) return XPBD_OK;
-    with_lanes(n, [&](auto g) {
+    with_lanes(n, n_btris, [&](auto g) {
         constexpr int G = decltype(g)::value;
         k_bone_bind<G><<<bone_ctas(n, G), kBoneThreads, 0, (cudaStream_t)stream>>>(
             n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(bone4), n_btris, btris,
@@ -444,7 +449,7 @@ int xpbd_bone_slide_targets(int32_t n, const float* muscle4, const int32_t* anch
         reinterpret_cast<const float4*>(bone4), n_btris, btris, reinterpret_cast<float4*>(pin_target),               \
         reinterpret_cast<float4*>(attach_target)
     if (reproject)
-        with_lanes(n, [&](auto g) {
+        with_lanes(n, n_btris, [&](auto g) {
             constexpr int G = decltype(g)::value;
             k_bone_slide_targets<true, G><<<bone_ctas(n, G), kBoneThreads, 0, s>>>(XPBD_SLIDE_ARGS);
         });
@@ -474,7 +479,7 @@ int xpbd_surface_bind(int32_t n, const float* query4, int32_t n_sverts, const fl
     if (!a16(query4) || !a16(surf4) || !a8(out_uv))
         return fail(XPBD_ERR_ALIGN, "xpbd_surface_bind: [n][4] arrays 16-byte, uv 8-byte aligned");
     if (n == 0) return XPBD_OK;
-    with_lanes(n, [&](auto g) {
+    with_lanes(n, n_stris, [&](auto g) {
         constexpr int G = decltype(g)::value;
         k_surface_bind<G><<<bone_ctas(n, G), kBoneThreads, 0, (cudaStream_t)stream>>>(
             n, reinterpret_cast<const float4*>(query4), reinterpret_cast<const float4*>(surf4), n_stris, stris,

@@ -255,3 +255,46 @@ def test_more_queries_than_32_bit_threads():
         assert abs(float(loc[k, 2]) - 0.5) < 1e-6 and float(uv[k, 0]) > 0.0
     del q4, face, uv, loc
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("n,nf", [(24_000, 24), (24_999, 24), (25_000, 24), (60_000, 59), (60_000, 61)])
+def test_few_faces_agree_with_many_lanes(n, nf):
+    """One lane per query where the faces are few against the queries: the same
+    faces, coordinates and offsets, bit for bit, as the same queries get in
+    small calls (32 lanes), in the bindings and in the re-projection."""
+    lib = capi.load()
+    v, t, _ = _bones()
+    t = np.ascontiguousarray(t[:nf])
+    rng = np.random.default_rng(nf)
+    q4 = _d(_v4((v[t[rng.integers(0, nf, n), 0]] + rng.normal(scale=0.01, size=(n, 3))).astype(np.float32)))
+    b4, td = _d(_v4(v)), _d(t)
+    nv, far = v.shape[0], C.c_float(0.012)
+
+    def buffers():
+        return (torch.full((n,), -7, dtype=torch.int32, device="cuda"), torch.full((n, 2), -7.0, device="cuda"),
+                torch.full((n, 4), -7.0, device="cuda"), torch.full((n,), -7.0, device="cuda"),
+                torch.full((n,), -7, dtype=torch.int32, device="cuda"))
+
+    def run(step):
+        face, uv, loc, gap, ok = buffers()
+        sface, suv, pin = torch.empty_like(face), torch.empty_like(uv), torch.zeros_like(loc)
+        moved = (q4 + torch.tensor([0.003, -0.002, 0.001, 0.0], device="cuda")).contiguous()
+        for k in range(0, n, step):
+            m = min(step, n - k)
+            assert lib.xpbd_bone_bind(m, _p(q4[k:]), nv, _p(b4), nf, _p(td), far, _p(face[k:]), _p(uv[k:]), _p(loc[k:]),
+                                      None) == 0
+        bf, buv, bl = face.clone(), uv.clone(), loc.clone()
+        for k in range(0, n, step):
+            m = min(step, n - k)
+            assert lib.xpbd_bone_slide_targets(m, _p(moved[k:]), _p(face[k:]), _p(uv[k:]), _p(bf[k:]), _p(buv[k:]),
+                                               _p(bl[k:]), C.c_float(0.004), 1, far, nv, _p(b4), nf, _p(td),
+                                               _p(pin[k:]), None, None) == 0
+            assert lib.xpbd_surface_bind(m, _p(q4[k:]), nv, _p(b4), nf, _p(td), far, _p(sface[k:]), _p(suv[k:]),
+                                         _p(gap[k:]), _p(ok[k:]), None) == 0
+        torch.cuda.synchronize()
+        return face, uv, loc, bf, buv, bl, pin, sface, suv, gap, ok
+
+    whole, parts = run(n), run(2000)
+    assert 0 < int(whole[-1].sum()) < n  # some within reach, some not
+    for a, b in zip(whole, parts):
+        assert torch.equal(a, b)
