@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import weakref
 from pathlib import Path
 
 import numpy as np
@@ -56,6 +57,43 @@ def scene_from_cfg(cfg: dict) -> Scene:
         from .meshgen import batched_box_scene
         return batched_box_scene(**syn)
     raise ValueError(f"unknown synthetic scene kind {kind!r}")
+
+
+class _LaunchValues:
+    """The values that a frame's launches take from the host objects ``parts``:
+    their numbers, texts, tuples, tensors (by identity) and parameter structs.
+    A captured frame holds them as they were; ``same`` says whether they still
+    are.  Two list comparisons per object, about 20 us for a simulator, where
+    the launches of an eager frame take milliseconds."""
+
+    #: attributes that change from frame to frame and that no launch reads
+    BOOKKEEPING = frozenset({"step_cnt", "slide_interval", "_frame_loaded", "_reproject", "_status_pending",
+                             "_accum_dirty", "_n_broad", "_peak", "_program_sub", "_freeze_warned", "_captured"})
+
+    def __init__(self, parts: list):
+        self.rows = []
+        for p in parts:
+            d = p.__dict__
+            names = [k for k, v in d.items() if k not in self.BOOKKEEPING
+                     and (v is None or isinstance(v, (int, float, str, tuple, np.generic, torch.Tensor)))]
+            structs = [k for k, v in d.items() if isinstance(v, C.Structure)]
+            self.rows.append((weakref.ref(p), len(d), names, [d[k] for k in names], structs,
+                              [bytes(d[k]) for k in structs]))
+
+    @staticmethod
+    def _differ(a, b) -> bool:
+        return a is not b and (type(a) is not type(b) or isinstance(a, torch.Tensor) or bool(a != b))
+
+    def same(self, parts: list) -> bool:
+        if len(parts) != len(self.rows):
+            return False
+        for p, (ref, n, names, values, structs, contents) in zip(parts, self.rows):
+            d = p.__dict__
+            if (ref() is not p or len(d) != n or any(map(self._differ, map(d.get, names), values))
+                    or any(not isinstance(d.get(k), C.Structure) or bytes(d[k]) != c
+                           for k, c in zip(structs, contents))):
+                return False
+        return True
 
 
 class MultiGridSim(MuscleSim):
@@ -302,6 +340,7 @@ class MultiGridSim(MuscleSim):
             self.dcd = UdcfDcdCollider(self, sc.surface_tris, prm)
             self.collision_solvers_iter.append(self.dcd.solve)
         self._frame_loaded = None
+        self._captured = None  # what the captured sliding frames were given
 
     # ----------------------------------------------------------- kinematics
     def _cons_targets(self, frame: int) -> np.ndarray:
@@ -794,12 +833,37 @@ class MultiGridSim(MuscleSim):
                 and all(getattr(c, "graph_safe", False) for c in cs) and len(cs) <= 1
                 and getattr(self, "program", None) is None)
 
+    def _launch_parts(self) -> list:
+        """The objects that a frame's launches take values from."""
+        dcd = getattr(self, "dcd", None)
+        parts = [self, self.mg, getattr(self.mg, "coarse", None), self.fascia, getattr(self.fascia, "solver", None), dcd,
+                 getattr(dcd, "buf", None), getattr(dcd, "params", None), *self.collision_solvers]
+        return [p for p in parts if p is not None] + [getattr(fn, "__self__", fn) for fn in self.collision_solvers_iter]
+
+    def _graph_frame(self) -> None:
+        """The frame as a captured graph.  Sliding frames need two, with and
+        without the re-projection of the binding, and follow the simulator's
+        parameters: both are captured again when one has changed (captured
+        frames of the other modes keep theirs until release_graphs())."""
+        if self.use_sliding and self.use_graphs:
+            parts = self._launch_parts()
+            if self._captured is not None and not self._captured.same(parts):
+                self._stream.synchronize()
+                self.release_graphs()
+                self._captured = None
+            self._graph(("frame", self._reproject), self._frame_fused)
+            if self._captured is None:
+                self._captured = _LaunchValues(parts)
+            return
+        self._graph(("frame", self._reproject), self._frame_fused)
+
     def _frame_fused(self) -> None:
         self._targets_kernel()
         if self.fascia is not None:
             self.fascia.advect()  # step_frame (mg.py:1413-1416): once per frame, before the substeps
         if self.mg is not None:
             self.mg.refresh_target()
+        mg = self.mg if self.use_multigrid else None
         sdf = self.collision_solvers[0] if self.collision_solvers else None
         if sdf is not None:
             sdf.bake()
@@ -810,16 +874,16 @@ class MultiGridSim(MuscleSim):
         self.apply_pintotarget_all()
         vel = 0 if self.quasi_static else capi.OP_VELOCITY
         push = capi.OP_SDF if sdf is not None else 0
-        if self.mg is None and self.fascia is None and not self.n_m2m and not self.collision_solvers_iter:
+        if mg is None and self.fascia is None and not self.n_m2m and not self.collision_solvers_iter:
             if self._fused_substeps(self.nsubsteps, self.fine_iters, capi.OP_PREDICT | pin,
                                     capi.OP_PREDICT | pin | push | vel, push | vel):
                 return
         for sub in range(self.nsubsteps):
-            if self.mg is None:
+            if mg is None:
                 self._vstep(capi.OP_PREDICT | pin | ((push | vel) if sub > 0 else 0))
             else:
                 self._vstep(capi.OP_PREDICT | ((push | vel) if sub > 0 else 0))
-                self.mg.vcycle(pin_fine=bool(pin))
+                mg.vcycle(pin_fine=bool(pin))
             self._substep_iterations()
             if self.fascia is not None:  # post_phase (mg.py:1361-1364), before the push-out and velocity
                 self.fascia.substep()
@@ -862,8 +926,7 @@ class MultiGridSim(MuscleSim):
         if self._frame_loaded != frame:
             self.load_frame_targets(frame)
         if self._program_fusable():
-            # frames that re-project the slide binding launch another targets kernel
-            self._graph(("frame", self._reproject), self._frame_fused)
+            self._graph_frame()
         else:
             self._kinematic_step(frame)
             if self.fascia is not None:

@@ -298,3 +298,101 @@ def test_few_faces_agree_with_many_lanes(n, nf):
     assert 0 < int(whole[-1].sum()) < n  # some within reach, some not
     for a, b in zip(whole, parts):
         assert torch.equal(a, b)
+
+
+def _slide_sim(interval, cls=None, **over):
+    from rlmusclev2_b200.mg import MultiGridSim, load_config
+    from rlmusclev2_b200.meshgen import humanv2_scene
+    cfg = load_config("rlmusclev2_b200/configs/humanv2_synth.json")
+    cfg["demo"]["collision"]["sdf_res"] = 64
+    cfg.update(target_mode="mesh", use_sliding=True, slide_interval=interval, fine_iterations=3, **over)
+    sc = humanv2_scene(seed=2, n_muscles=4, n_bones=4, target_tets=9000, fascia_tets=1500, box=(0.3, 0.3, 0.3))
+    return (cls or MultiGridSim)(cfg, scene=sc), sc
+
+
+def _slide_state(sim):
+    sim.synchronize()
+    return [sim.positions_np(), sim._bind_face.cpu().numpy(), sim._bind_uv.cpu().numpy(), sim._local4.cpu().numpy(),
+            sim._pin_tgt.cpu().numpy()]
+
+
+@pytest.mark.parametrize("interval", [1, 2, 3])
+def test_sliding_graphs_match_eager_launches_and_the_phase_program(interval):
+    """Sliding frames replayed from their graphs (two when only some frames
+    re-project) against the same launches issued eagerly, bit for bit (the
+    sums between tiles are integers), and against the phase program of unfused
+    primitives: positions within 1e-4 m, the frame gate of the parity tests
+    (sums in another order; the faces are not compared there, since noise of
+    3e-8 m on the positions gives one bound vertex in ten another of two faces
+    that share its closest point)."""
+    graph, sc = _slide_sim(interval)
+    eager, _ = _slide_sim(interval)
+    phase, _ = _slide_sim(interval)
+    eager.use_graphs = False
+    phase.build_program()
+    moved = 0
+    for frame in range(1, 8):
+        before = graph._bind_uv.clone()
+        for s in (graph, eager, phase):
+            s.set_fiber_activation(sc.activation(frame))
+            s.step_frame(frame)
+        a, b, c = (_slide_state(s) for s in (graph, eager, phase))
+        moved += int((graph._bind_uv != before).any())
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
+        assert np.abs(a[0] - c[0]).max() <= 1e-4
+    assert set(graph._graphs) == {("frame", True)} | ({("frame", False)} if interval > 1 else set())
+    # the re-projecting frames move the binding, the others and frame 1 (the pose it was bound in) do not
+    assert moved == len(range(1, 8, interval)) - 1
+    assert np.abs(a[0] - sc.verts).max() > 1e-3
+
+
+def _no_slide(s):
+    s.slide_range = 0.0
+
+
+def _more_iterations(s):
+    s.fine_iters = 5
+
+
+def _fewer_substeps(s):
+    s.nsubsteps = 6
+
+
+def _soft_pin(s):
+    s.presubframe_pintotarget = 0.25
+
+
+def _heavier(s):
+    s._prm.gravity[1] = -9.8
+
+
+def _wide_push_out(s):
+    # the muscles lie 31 mm off the bones at least
+    s.collision_solvers[0].band = 0.08
+    s.collision_solvers[0]._s.contact_offset = 0.04
+
+
+@pytest.mark.parametrize("change", [_no_slide, _more_iterations, _fewer_substeps, _soft_pin, _heavier,
+                                    _wide_push_out])
+def test_sliding_frames_follow_their_parameters(change):
+    """A parameter set between two sliding frames counts from the next frame
+    on, captured or not."""
+    graph, sc = _slide_sim(2)
+    eager, _ = _slide_sim(2)
+    kept, _ = _slide_sim(2)
+    eager.use_graphs = False
+    for frame in range(1, 7):
+        if frame == 4:
+            change(graph)
+            change(eager)
+        for s in (graph, eager, kept):
+            s.set_fiber_activation(sc.activation(frame))
+            s.step_frame(frame)
+        if frame in (1, 2, 4):
+            captured = graph._graphs[("frame", frame % 2 == 1)].value
+        elif frame == 6:  # captured once per change, not every frame
+            assert graph._graphs[("frame", False)].value == captured
+    for x, y in zip(_slide_state(graph), _slide_state(eager)):
+        np.testing.assert_array_equal(x, y)
+    assert np.abs(_slide_state(graph)[0] - _slide_state(kept)[0]).max() > 0
