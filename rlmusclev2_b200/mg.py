@@ -845,6 +845,8 @@ class MultiGridSim(MuscleSim):
         without the re-projection of the binding, and follow the simulator's
         parameters: both are captured again when one has changed (captured
         frames of the other modes keep theirs until release_graphs())."""
+        if self._accum_dirty:  # unfused primitives have left sums behind
+            self.clear()
         if self.use_sliding and self.use_graphs:
             parts = self._launch_parts()
             if self._captured is not None and not self._captured.same(parts):
