@@ -831,7 +831,17 @@ class MultiGridSim(MuscleSim):
         dcd = getattr(self, "dcd", None)
         return (all(dcd is not None and fn == dcd.solve for fn in its) and not getattr(self, "constraint_solvers", None)
                 and all(getattr(c, "graph_safe", False) for c in cs) and len(cs) <= 1
-                and getattr(self, "program", None) is None)
+                and getattr(self, "program", None) is None
+                and not (getattr(self, "use_sliding", False) and self._own_phases()))
+
+    #: what the phase program calls on the simulator
+    _PHASES = ("build_program", "substep", "integrate", "clear", "solve_constraints", "apply_dP", "apply_pintotarget",
+               "apply_pintotarget_all", "update_velocities")
+
+    def _own_phases(self) -> bool:
+        """A subclass or the instance has replaced a part of the phase program."""
+        t = type(self)
+        return any(getattr(t, n) is not getattr(MultiGridSim, n) or n in self.__dict__ for n in self._PHASES)
 
     def _launch_parts(self) -> list:
         """The objects that a frame's launches take values from."""

@@ -418,3 +418,21 @@ def test_sliding_frames_start_from_empty_sums():
     a, b = (s.positions_np() for s in sims)
     print("difference", np.abs(a - b).max())
     assert np.abs(a - b).max() <= 1e-4  # boundary sums are float atomics here
+
+
+def test_sliding_frames_run_a_replaced_phase_program():
+    """A subclass's own phases run, frame after frame."""
+    from rlmusclev2_b200.mg import MultiGridSim
+
+    class Counting(MultiGridSim):
+        calls = 0
+
+        def update_velocities(self):
+            self.calls += 1
+            super().update_velocities()
+
+    sim, sc = _slide_sim(1, cls=Counting)
+    for frame in (1, 2):
+        sim.set_fiber_activation(sc.activation(frame))
+        sim.step_frame(frame)
+    assert sim.calls == 2 * sim.nsubsteps
