@@ -12,6 +12,7 @@ from pathlib import Path
 MAX_MATERIALS = 64
 MAX_ATTACH_MATERIALS = 16
 MAX_TILE_VERTS = 4096
+FRAME_MAX_ITERS = 1 << 20  # n_sub x n_iters of one xpbd_frame_persistent
 NOALLOC_MAX_VERTS = 262144
 
 OK = 0

@@ -475,11 +475,13 @@ class XpbdEngine:
     def _fused_substeps(self, n_sub: int, n_iters: int, first_ops: int, sub_ops: int, last_ops: int) -> bool:
         """n_sub substeps of (vertex step, n_iters fused iterations) and the
         last vertex step, in one persistent launch per tile range; False (and
-        nothing launched) where the tiles do not fit at once or the tile
-        variant asks for an instance the frame pass does not have."""
+        nothing launched) where the tiles do not fit at once, the iterations
+        are none or more than a launch takes, or the tile variant asks for an
+        instance the frame pass does not have."""
         if not (self.use_persistent and self._persist_fits and self.fused_mode == capi.PROJECT_FUSED
                 and self.persistent_sync == "exchange" and self._exchange is not None
-                and n_iters > 0 and self.n_cons > 0) or (self._prm.tile_variant & ~0x53):
+                and 0 < n_sub * n_iters <= capi.FRAME_MAX_ITERS
+                and self.n_cons > 0) or (self._prm.tile_variant & ~0x53):
             return False
         f = capi.XpbdFrame()
         f.n_sub, f.n_iters, f.ex = int(n_sub), int(n_iters), C.addressof(self._exchange)

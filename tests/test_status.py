@@ -8,7 +8,7 @@ copies the words behind every frame and raises at the next frame or
 synchronising read; these tests pin which bits are fatal.
 """
 from rlmusclev2_b200 import _capi as capi
-from rlmusclev2_b200.engine import status_error
+from rlmusclev2_b200.engine import XpbdEngine, status_error
 
 
 def test_clean_words_pass():
@@ -38,3 +38,27 @@ def test_dcd_sort_timeout_is_fatal():
 def test_all_fatal_bits_reported_together():
     msg = status_error(capi.STATUS_BARRIER_TIMEOUT | capi.STATUS_ACC_RANGE, capi.STATUS_BARRIER_TIMEOUT)
     assert msg.count(";") == 2
+
+
+class _FrameEngine:
+    """What _fused_substeps reads of an engine, with a library that counts launches."""
+    use_persistent, _persist_fits, persistent_sync, n_cons = True, True, "exchange", 1
+    fused_mode = capi.PROJECT_FUSED
+
+    def __init__(self):
+        self._prm, self._tiles, self._verts = capi.XpbdParams(), capi.XpbdTiles(), capi.XpbdVerts()
+        self._exchange, self._persist, self._sdf, self._sp = capi.XpbdExchange(), [capi.XpbdPersist()] * 2, None, None
+        self.launched = []
+        self._lib = type("Lib", (), {"xpbd_frame_persistent": lambda _, p, t, v, ps, f, s: self.launched.append(
+            (f._obj.n_sub, f._obj.n_iters)) or 0})()
+
+
+def test_frames_that_one_launch_does_not_take_go_substep_by_substep():
+    """No substeps, no iterations, or more iterations in all than one launch
+    takes: nothing is launched and the caller runs the substeps one by one, as
+    many iterations each as before."""
+    for n_sub, n_iters, fits in ((10, 20, True), (1, 1 << 20, True), (0, 20, False), (3, 0, False),
+                                 (2, (1 << 19) + 1, False), (10, 1 << 20, False), (1, (1 << 20) + 1, False)):
+        e = _FrameEngine()
+        assert XpbdEngine._fused_substeps(e, n_sub, n_iters, 0, 0, 0) is fits
+        assert e.launched == ([(n_sub, n_iters)] * 2 if fits else [])
