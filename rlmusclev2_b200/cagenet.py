@@ -126,7 +126,7 @@ class CageMLP:
         transpose when a backward follows).  train=False writes only the
         outputs (no pre-activations, no transposed activations).  Returns
         Y[:m, :3] (a view)."""
-        p = self._mlp(m)
+        p = self._mlp(self.m_pad)  # every row of the buffers, whatever slice of them is returned
         if train:
             p.z[:] = [t.data_ptr() for t in self.Z]
             p.ht[:] = [t.data_ptr() for t in self.Ht[1:]]

@@ -226,3 +226,18 @@ def test_fused_backward_equals_layer_launches(m):
             d, dt, k = dn, dnt, 256
     torch.cuda.synchronize()
     assert int(net.status.item()) == 0
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_forward_returns_the_slice_that_was_asked_for(train):
+    """forward computes every row of its buffers; m only says which outputs to
+    return, and slices as anywhere else (past the end, from the end)."""
+    net = CageMLP("cuda:0", 300)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    net.X.copy_(torch.randn(net.X.shape, generator=g, device="cuda"))
+    whole = net.forward(net.m_pad, train=train).clone()
+    assert whole.shape == (384, 3) and float(whole.abs().min()) > 0
+    for m in (0, 1, 300, 384, 1000, -84, None):
+        net.Y.zero_()
+        assert torch.equal(net.forward(m, train=train), whole[:m])
+    assert int(net.status.item()) == 0
