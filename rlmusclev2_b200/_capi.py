@@ -7,6 +7,8 @@ Python or CPU implementation.
 from __future__ import annotations
 
 import ctypes as C
+import functools
+import zlib
 from pathlib import Path
 
 MAX_MATERIALS = 64
@@ -247,6 +249,12 @@ def load(build_if_missing: bool = False) -> C.CDLL:
         fn.restype = res
     _LIB = lib
     return lib
+
+
+@functools.lru_cache(maxsize=1)
+def build_tag() -> str:
+    """Checksum of the library file: timings kept on disk belong to one build."""
+    return f"{zlib.crc32(lib_path().read_bytes()):08x}"
 
 
 def exported_symbols() -> list[str]:

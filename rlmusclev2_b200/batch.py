@@ -10,8 +10,8 @@ batched SDF bake, 10 substeps) replays as one captured CUDA graph.
 
 ``autotune()`` times the tet-pass configurations on the live batch (tile size,
 CTAs per SM, persistent ranges vs per-iteration launches, tet-stream prefetch)
-and keeps the fastest; results are cached per (GPU, mesh, material set) in a
-JSON file.
+and keeps the fastest; results are cached per (GPU, library build, mesh,
+material set, iterations) in a JSON file.
 """
 from __future__ import annotations
 
@@ -108,30 +108,51 @@ class BatchSim(MultiGridSim):
                 dict(persistent=False, variant=32), dict(persistent=False, variant=33),
                 dict(persistent=False, variant=96), dict(persistent=False, variant=97)]
 
-    def _time_iterations(self, n_iters: int, reps: int) -> float:
-        """ms per Jacobi iteration with the frame's own grouping: ``reps``
-        calls of n_iters fused iterations (n_iters = fine_iterations)."""
+    def _time_ms(self, body, reps: int) -> float:
+        """Median ms of ``reps`` calls of body after one that is not timed, each
+        call on the state that the one before left."""
         s = self._stream
-        self._fused_iterations(n_iters)
+        body()
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(reps + 1)]
+        ev[0].record(s)
+        for e in ev[1:]:
+            body()
+            e.record(s)
         s.synchronize()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(s)
-        for _ in range(reps):
-            self._fused_iterations(n_iters)
-        e1.record(s)
-        e1.synchronize()
-        return e0.elapsed_time(e1) / (reps * n_iters)
+        return float(np.median([a.elapsed_time(b) for a, b in zip(ev[:-1], ev[1:])]))
+
+    def _time_candidate(self) -> float:
+        """ms per Jacobi iteration of the current configuration: of whole frames
+        as step_frame replays them (the one-launch frame, or the launches per
+        substep with their vertex steps), at the loaded pose and without
+        re-projection: by their bare iterations the candidates came out in
+        another order, and the pick's frames were 4 to 6 % slower than the
+        best's at 40, 64 and 256 instances.  With parts that keep a state of their own between
+        frames (multigrid, fascia, hooks), of the iterations by themselves."""
+        n = self.nsubsteps * self.fine_iters
+        if (self.mg is not None or self.fascia is not None or self.collision_solvers_iter or n <= 0
+                or not self._program_fusable()):
+            it = max(1, self.fine_iters)
+            return self._time_ms(lambda: self._fused_iterations(it), 5) / it
+        reproject, self._reproject = self._reproject, False
+        try:
+            return self._time_ms(lambda: self._graph("tune", self._frame_fused), 5) / n
+        finally:
+            self._stream.synchronize()
+            self.release_graphs()  # captured for this candidate
+            self._reproject = reproject
 
     def _tune_key(self) -> str:
         name = torch.cuda.get_device_name(self.device)
         flags = sorted({int(m["flags"]) for m in self.layout.materials})
         cands = len(self._candidates())
-        return f"{name}|nv={self.NV}|nt={self.NT}|inst={self.n_inst}|flags={flags}|iters={self.fine_iters}|cands={cands}"
+        return (f"{name}|lib={capi.build_tag()}|nv={self.NV}|nt={self.NT}|inst={self.n_inst}|flags={flags}"
+                f"|sub={self.nsubsteps}|iters={self.fine_iters}|cands={cands}")
 
     def autotune(self, use_cache: bool = True) -> dict:
         """Pick the fastest tet-pass configuration for this batch: persistent
         tile ranges (with or without tet-stream prefetch) or per-iteration
-        launches, timed on the current state (positions restored after)."""
+        launches, timed on frames from the current state (restored after)."""
         key = self._tune_key()
         cache = {}
         if use_cache and TUNE_CACHE.exists():
@@ -142,17 +163,21 @@ class BatchSim(MultiGridSim):
         if use_cache and key in cache:
             best = cache[key]
         else:
-            saved = self._pos4.clone()
+            if self._frame_loaded is None:
+                self.load_frame_targets(self.start_frame)
+            state = (self._pos4, self._prev4, self._vel4)
+            with torch.cuda.stream(self._stream):
+                saved = [t.clone() for t in state]
             results = []
             for c in self._candidates():
                 if c["persistent"] and not self._persist_fits:
                     continue
                 self.use_persistent = c["persistent"]
                 self._prm.tile_variant = c["variant"]
-                ms = self._time_iterations(self.fine_iters, max(3, 40 // self.fine_iters))
-                results.append((ms, c))
+                results.append((self._time_candidate(), c))
                 with torch.cuda.stream(self._stream):
-                    self._pos4.copy_(saved)
+                    for t, v in zip(state, saved):
+                        t.copy_(v)
             self._stream.synchronize()
             ms, best = min(results, key=lambda r: r[0])
             best = dict(best, ms_per_iteration=ms, tried=[dict(c, ms=m) for m, c in results])

@@ -156,3 +156,36 @@ def test_sdf_bake_runs_of_bricks(dims, n_caps):
     torch.cuda.synchronize()
     ref = O.sdf_bake(dims, origin, h, caps[:n_caps], None, band, "f32")
     np.testing.assert_allclose(phi.cpu().numpy(), ref, atol=2e-6, rtol=0)
+
+
+def test_autotune_times_frames_and_restores_the_state(monkeypatch):
+    """The candidates are timed on the frames that step_frame runs (whole
+    frames in one launch per range for the persistent one), the state is put
+    back, and a stored result belongs to one build, substep and iteration count."""
+    cfg = load_config(CFG)
+    sc = batched_box_scene(n_inst=5, seed=4, tets_lo=500, tets_hi=4000, sdf_res=32)
+    sim = BatchSim(cfg, scene=sc)
+    for f in (1, 2):
+        sim.step_frame_inputs(f)
+    sim.synchronize()
+    before = [t.clone() for t in (sim._pos4, sim._prev4, sim._vel4)]
+    calls = []
+    fused = sim._fused_substeps
+
+    def record(n_sub, n_iters, *ops):
+        calls.append((sim.use_persistent, int(sim._prm.tile_variant), n_sub, n_iters))
+        return fused(n_sub, n_iters, *ops)
+
+    monkeypatch.setattr(sim, "_fused_substeps", record)
+    best = sim.autotune(use_cache=False)
+    assert (True, 0, sim.nsubsteps, sim.fine_iters) in calls
+    assert {c["variant"] for c in best["tried"]} >= {0, 1, 32, 96}
+    for t, b in zip((sim._pos4, sim._prev4, sim._vel4), before):
+        assert torch.equal(t, b)
+    key = sim._tune_key()
+    assert capi.build_tag() in key
+    sim.nsubsteps += 1
+    assert sim._tune_key() != key
+    sim.nsubsteps -= 1
+    sim.step_frame_inputs(3)
+    assert np.isfinite(sim.positions_np()).all()
