@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "xpbd_round.cuh"
+
 namespace xpbd {
 
 struct M3 { float m[3][3]; };
@@ -20,15 +22,6 @@ __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return make_fl
 __device__ __forceinline__ float3 operator-(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
 __device__ __forceinline__ float3 operator-(float3 a) { return make_float3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ float3 operator*(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
-// a / s with one division: the products with the rounded reciprocal and a
-// residual step each, which rounds like three divisions (P. Markstein, 1990;
-// equal in all of 1.5e9 random pairs).  For finite a and s in [1e-30, 1e30].
-__device__ __forceinline__ float3 over(float3 a, float s) {
-    const float r = 1.f / s;
-    const float3 q = make_float3(a.x * r, a.y * r, a.z * r);
-    return make_float3(fmaf(fmaf(-q.x, s, a.x), r, q.x), fmaf(fmaf(-q.y, s, a.y), r, q.y),
-                       fmaf(fmaf(-q.z, s, a.z), r, q.z));
-}
 __device__ __forceinline__ float3 operator/(float3 a, float s) { return make_float3(a.x / s, a.y / s, a.z / s); }
 __device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ float3 cross(float3 a, float3 b) {
@@ -322,14 +315,6 @@ __device__ __forceinline__ float2 xpbd_consts(float k, float kd, float dt) {
         gamma = alpha * beta / dt;
     }
     return make_float2(alpha, gamma);
-}
-
-// x / 6, correctly rounded: one residual step on the product with the rounded
-// reciprocal (P. Markstein, 1990), three instructions instead of a division
-// (the residual is exact while |x| > 2^-100; volumes of 1e-30 m^3 are zero here).
-__device__ __forceinline__ float sixth(float x) {
-    const float q = x * (1.f / 6.f);
-    return fmaf(fmaf(-6.f, q, x), 1.f / 6.f, q);
 }
 
 __device__ __forceinline__ float3 sixth(float3 a) { return make_float3(sixth(a.x), sixth(a.y), sixth(a.z)); }
