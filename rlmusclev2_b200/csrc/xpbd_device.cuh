@@ -330,8 +330,18 @@ __device__ __forceinline__ bool con_volume(const float4 p[4], const float4* q, f
     g[1] = sixth(cross(d2, d0));
     g[2] = sixth(cross(d0, d1));
     g[3] = -((g[0] + g[1]) + g[2]);
-    const float ws = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
-    if (!(ws > 1e-9f)) return false;
+    float ws = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
+    if (!(ws > 1e-9f)) {
+        if (ws == ws) return false;
+        // not a number: where the products overflowed, the divisions keep the
+        // infinities, and the range check sees the corrections
+        g[0] = cross(d1, d2) / 6.f;
+        g[1] = cross(d2, d0) / 6.f;
+        g[2] = cross(d0, d1) / 6.f;
+        g[3] = -((g[0] + g[1]) + g[2]);
+        ws = p[0].w * dot(g[0], g[0]) + p[1].w * dot(g[1], g[1]) + p[2].w * dot(g[2], g[2]) + p[3].w * dot(g[3], g[3]);
+        if (!(ws > 1e-9f)) return false;
+    }
     const float volume = sixth(dot(cross(d0, d1), d2));
     const float C = volume - V0;
     float dsum = 0.f, gamma = 1.f;

@@ -166,3 +166,24 @@ def test_deferred_svd_pass_is_bit_identical(case):
         assert np.isfinite(out[0]).all()
         assert np.array_equal(out[0], out[1]), (case, persistent)
         assert np.abs(out[0] - deformed).max() > 0
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_volume_of_an_overflowing_tet_is_reported(fused):
+    """A tet of 1e20 m has infinite volume gradients: its corrections are not
+    numbers, and the range check says so instead of leaving the term out."""
+    from rlmusclev2_b200 import _capi as capi
+    from rlmusclev2_b200.builder import collect_raw_constraints, lumped_mass
+    verts = np.float32([[1, 0, 0], [0, 1, 0], [0, 0, 1], [0, 0, 0]])
+    tets = np.int32([[0, 1, 2, 3]])
+    table = collect_raw_constraints(verts, tets, [dict(type="volume", name="v", stiffness=1e6,
+                                                       dampingratio=0.0)]).sorted_by_type()
+    sim = XpbdSolver(verts, tets, table, mass=lumped_mass(verts, tets, 1000.0)[0], dt=1.0 / 240.0, device="cuda:0")
+    sim._fused_iterations(1)
+    assert sim.persistent_status() == 0
+    sim.set_positions(verts * np.float32(1e20))
+    if fused:
+        sim._fused_iterations(1)
+    else:
+        sim._fused_iteration()
+    assert sim.persistent_status() & capi.STATUS_ACC_RANGE
