@@ -72,3 +72,47 @@ def test_network_in_a_fresh_thread():
     torch.cuda.synchronize()
     assert int(net.status.item()) == 0
     assert float(net.loss.item()) == 600.0  # features and biases are zero, so are the outputs
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_two_simulators_at_once(graphs):
+    """Two engines stepped and read by two threads on their own streams give,
+    bit for bit, what each gives alone: the one-launch frames of one do not
+    disturb the other's (their tiles wait for one another within a grid only)."""
+    dims = [(8, 8, 32), (5, 7, 41)]
+    alone = []
+    for d in dims:
+        s = _box(dims=d)
+        s.use_graphs = graphs
+        for _ in range(60):
+            s.step()
+        alone.append(s.positions_np())
+    sims = [_box(dims=d) for d in dims]
+    reads = [[], []]
+
+    def run(k):
+        def job():
+            sims[k].use_graphs = graphs
+            for f in range(60):
+                sims[k].step()
+                if f % 3 == 0:
+                    reads[k].append(sims[k].positions_np())
+        return job
+
+    _in_threads([run(0), run(1)])
+    for s, ref, r in zip(sims, alone, reads):
+        assert s.persistent_status() == 0
+        np.testing.assert_array_equal(s.positions_np(), ref)
+        assert len({x.ctypes.data for x in r}) == len(r)  # every read an array of its own
+
+
+def test_one_engine_read_by_two_threads():
+    """positions_np from two threads on one engine: both read the same positions."""
+    s = _box()
+    for _ in range(3):
+        s.step()
+    ref = s.positions_np()
+    out = [[], []]
+    _in_threads([lambda k=k: out[k].extend(s.positions_np() for _ in range(50)) for k in (0, 1)])
+    for x in out[0] + out[1]:
+        np.testing.assert_array_equal(x, ref)
