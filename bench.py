@@ -363,15 +363,30 @@ def run_ours(args):
         ms_e2e = float(t.item())
 
     # ---- roofline of the dominant kernel, measured inside a real frame: one
-    # frame replayed launch by launch with events around every Jacobi iteration
-    # (tile pass + boundary finish) on the engine stream.
+    # frame replayed launch by launch with events around its tet passes on the
+    # engine stream (the launch of all substeps where the frame is one; else
+    # every substep's iterations, or every iteration with its boundary finish).
     L = sim.layout
     flush_l2()
     frame_resident(nf - 1)
     iters = []
     sim._targets_kernel()
     sim.collision_solvers[0].bake() if sim.collision_solvers else None
-    for sub in range(sim.nsubsteps):
+    pin = capi.OP_PIN if sim._has_pins else 0
+    vel = (0 if sim.quasi_static else capi.OP_VELOCITY) | (capi.OP_SDF if sim.collision_solvers else 0)
+    whole = False
+    if sim.mg is None and sim.fascia is None and not sim.n_m2m and not sim.collision_solvers_iter:
+        if pin:
+            sim._vstep(capi.OP_PIN)
+        sim.apply_pintotarget_all()
+        a, b = ev(), ev()
+        a.record(stream)
+        whole = sim._fused_substeps(sim.nsubsteps, sim.fine_iters, capi.OP_PREDICT | pin,
+                                    capi.OP_PREDICT | pin | vel, vel)
+        b.record(stream)
+        if whole:
+            iters.append((a, b, sim.nsubsteps * sim.fine_iters))
+    for sub in range(0 if whole else sim.nsubsteps):
         sim._vstep(capi.OP_PREDICT | (capi.OP_PIN if sim._has_pins and sim.mg is None else 0))
         if sim.mg is not None:
             sim.mg.vcycle(pin_fine=sim._has_pins)
@@ -419,10 +434,9 @@ def run_ours(args):
         every = max(1, int(sim.dcd.params.bvh_rebuild_every))
         per_sub += sum(sim.dcd.buf.broadphase_launches(True, refit_only=(k % every) != 0)
                        for k in range(sim.nsubsteps)) / sim.nsubsteps
-    # all substeps in one launch per tile range, else a vertex step ends the frame
     frame_kernel = bool(persistent and sim.persistent_sync == "exchange" and sim._exchange is not None
                         and not (sim._prm.tile_variant & ~0x53))
-    whole = frame_kernel and sim.mg is None and sim.fascia is None and not sim.n_m2m
+    # one launch per tile range, or the substeps' launches and a vertex step at the end
     launches_per_frame = 1 + (1 if sim.collision_solvers else 0) + (1 if sim._has_pins else 0) + (
         1 if sim.mg is not None else 0) + (len(sim._persist) if whole else sim.nsubsteps * per_sub + 1)
     n_iter = sim.nsubsteps * sim.fine_iters

@@ -116,3 +116,26 @@ def test_one_engine_read_by_two_threads():
     _in_threads([lambda k=k: out[k].extend(s.positions_np() for _ in range(50)) for k in (0, 1)])
     for x in out[0] + out[1]:
         np.testing.assert_array_equal(x, ref)
+
+
+def test_positions_are_read_on_the_engines_own_device(monkeypatch):
+    """The read-back launches its gather with the engine's stream, and so its
+    device, current: the caller may have another one selected."""
+    s = _box()
+    s.step()
+    lib, current = s._lib, []
+
+    class Lib:
+        def __getattr__(self, name):
+            if name == "xpbd_gather":
+                current.append(torch.cuda.current_stream() == s._stream)
+            return getattr(lib, name)
+
+    monkeypatch.setattr(s, "_lib", Lib())
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):  # what the caller queued on its own stream is waited for
+        torch.cuda._sleep(20_000_000)
+        s._pos4[:, :3] += 1.0
+        x = s.positions_np()
+    assert current == [True]
+    np.testing.assert_array_equal(x, s._pos4[:, :3].cpu().numpy()[s.layout.inv])
