@@ -164,6 +164,7 @@ class XpbdEngine:
         # host copies of the status words, queued behind every frame (see _post_status)
         self._status_host = torch.zeros(2, dtype=torch.int32).pin_memory()
         self._status_event = None
+        self._status_pending = False
         self._t_own = T(L.tile_own)
         self._build_exchange()
         self.use_persistent = True

@@ -68,7 +68,8 @@ class _LaunchValues:
 
     #: attributes that change from frame to frame and that no launch reads
     BOOKKEEPING = frozenset({"step_cnt", "slide_interval", "_frame_loaded", "_reproject", "_status_pending",
-                             "_accum_dirty", "_n_broad", "_peak", "_program_sub", "_freeze_warned", "_captured"})
+                             "_status_event", "_accum_dirty", "_n_broad", "_peak", "_program_sub", "_freeze_warned",
+                             "_captured"})
 
     def __init__(self, parts: list):
         self.rows = []

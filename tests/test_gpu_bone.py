@@ -436,3 +436,17 @@ def test_sliding_frames_run_a_replaced_phase_program():
         sim.set_fiber_activation(sc.activation(frame))
         sim.step_frame(frame)
     assert sim.calls == 2 * sim.nsubsteps
+
+
+def test_sliding_frames_are_captured_once(monkeypatch):
+    """Nothing that frames leave behind counts as a changed parameter."""
+    sim, sc = _slide_sim(1)
+    released = []
+    release = sim.release_graphs
+    monkeypatch.setattr(sim, "release_graphs", lambda: released.append(sim.step_cnt) or release())
+    for frame in range(1, 6):
+        sim.set_fiber_activation(sc.activation(frame))
+        sim.step_frame(frame)
+        sim.positions_np()
+        sim.metrics()
+    assert not released
