@@ -574,6 +574,7 @@ def run_box(args):
     alg = L.n_tets * 56 + L.n_verts * 40
     peak, peak_kind = _peak_hbm()
     it_s = ms * 1e-3 / 10
+    one = sim.use_persistent and sim._persist_fits and sim._exchange is not None  # the frame is one launch per range
     line = {
         "metric": "ms/frame", "value": round(ms, 4), "unit": "ms/frame", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms, 4), "higher_is_better": False, "scaling": "weak",
@@ -585,9 +586,10 @@ def run_box(args):
                 "d2h_bytes_per_step": L.n_verts * 12},
         "roofline": {"bound": "launch", "achieved": round(alg / it_s / 1e9, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(alg / it_s / 1e9 / peak, 5), "traffic": None, "peak_kind": peak_kind,
-                     "kernel": "whole substep (prediction, tile pass, boundary finish): launch-bound at 12k tets",
+                     "kernel": ("k_frame_tiles (a frame's ten substeps in one launch; launch and latency at 12k tets)" if one
+                                else "whole substep (prediction, tile pass, boundary finish): launch-bound at 12k tets"),
                      "algorithmic_bytes": alg},
-        "clocks": clk.summary(), "gpu_launches": int(21 * args.steps),
+        "clocks": clk.summary(), "gpu_launches": int((len(sim._persist) if one else 21) * args.steps),
     }
     sim.release_graphs()
     if world > 1:

@@ -37,7 +37,7 @@ enum {
 enum {
     XPBD_STATUS_PAIR_OVERFLOW = 1 << 0,    /* more candidate pairs than max_pairs (extra pairs dropped) */
     XPBD_STATUS_CONTACT_OVERFLOW = 1 << 1, /* more contacts than max_contacts (extra contacts dropped) */
-    XPBD_STATUS_STACK_OVERFLOW = 1 << 2,   /* BVH traversal deeper than its stack (query cut short) */
+    XPBD_STATUS_STACK_OVERFLOW = 1 << 2,   /* not set any more (the traversal has no stack) */
     XPBD_STATUS_BARRIER_TIMEOUT = 1 << 3,  /* a grid-wide wait of the persistent pass gave up (results invalid) */
     XPBD_STATUS_MMA_TIMEOUT = 1 << 4,      /* a tensor-core GEMM gave up waiting for its MMAs (results invalid) */
     XPBD_STATUS_ACC_RANGE = 1 << 5,        /* a tet correction left the fixed-point accumulator's safe range */

@@ -233,7 +233,7 @@ class DcdBuffers:
 class UdcfDcdCollider:
     """Self-collision DCD of a sim's surface triangles (movable vs movable with
     allow_self, the configuration of the synthetic humanV2 scene).  Register
-    ``solve`` in ``sim.collision_solvers_iter``: it rebuilds the LBVH on the
+    ``solve`` in ``sim.collision_solvers_iter``: it runs the broadphase on the
     first fine iteration of each substep and resolves contacts every
     iteration (udcf/solver.py:365-440)."""
 

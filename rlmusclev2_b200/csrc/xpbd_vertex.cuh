@@ -1,6 +1,6 @@
 // Per-vertex substep boundary (push-out out of the bones' grid SDF, velocity,
 // prediction, pin), shared by the per-vertex kernels (xpbd_core.cu) and the
-// persistent frame (xpbd_persist.cu).
+// persistent frame (xpbd_frame.cu).
 #pragma once
 #include "xpbd_common.cuh"
 #include "xpbd_device.cuh"
