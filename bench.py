@@ -393,7 +393,7 @@ def run_ours(args):
         if not sim.collision_solvers_iter:
             a, b = ev(), ev()
             a.record(stream)
-            sim._fused_iterations(sim.fine_iters)
+            sim._jacobi_iterations(sim.fine_iters)
             b.record(stream)
             iters.append((a, b, sim.fine_iters))
             continue

@@ -133,7 +133,7 @@ class BatchSim(MultiGridSim):
         if (self.mg is not None or self.fascia is not None or self.collision_solvers_iter or n <= 0
                 or not self._program_fusable()):
             it = max(1, self.fine_iters)
-            return self._time_ms(lambda: self._fused_iterations(it), 5) / it
+            return self._time_ms(lambda: self._jacobi_iterations(it), 5) / it
         reproject, self._reproject = self._reproject, False
         try:
             return self._time_ms(lambda: self._graph("tune", self._frame_fused), 5) / n

@@ -303,7 +303,7 @@ class LearnedWarmStart:
                                                   self.sp))
 
     def iterate(self, n: int) -> None:
-        self.sim._fused_iterations(n)
+        self.sim._jacobi_iterations(n)
 
     def restrict_final(self) -> None:
         """Cage state <- restrict(final fine state) (prior: the current cage)."""

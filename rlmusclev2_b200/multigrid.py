@@ -208,14 +208,14 @@ class DeviceMultigrid:
                                                    C.c_void_p(self.pin4.data_ptr()), s._sp))
         if self.beta != 0.0:
             for _ in range(self.iters):  # ARAP sweep, then the soft attach (mg.py:1057-1062)
-                co._fused_iterations(1)
+                co._jacobi_iterations(1)
                 capi.check(s._lib.xpbd_blend_to_target(int(self.attach_idx.shape[0]),
                                                        C.c_void_p(self.attach_idx.data_ptr()), co.n_verts,
                                                        C.c_void_p(co._pos4.data_ptr()),
                                                        C.c_void_p(self.pin4.data_ptr()), C.c_float(self.beta),
                                                        s._sp))
         else:
-            co._fused_iterations(self.iters)
+            co._jacobi_iterations(self.iters)
         capi.check(s._lib.xpbd_mg_prolong_delta(C.byref(self.g), C.c_void_p(co._pos4.data_ptr()),
                                                 C.c_void_p(self.prev.data_ptr()), C.c_void_p(s._pos4.data_ptr()),
                                                 C.c_void_p(vf) if vf else None, C.c_void_p(pt) if pt else None,

@@ -450,3 +450,22 @@ def test_sliding_frames_are_captured_once(monkeypatch):
         sim.positions_np()
         sim.metrics()
     assert not released
+
+
+def test_sliding_multigrid_follows_its_switch():
+    """use_multigrid set to False between sliding frames leaves the V-cycle out, captured or not."""
+    over = dict(use_multigrid=True, mg_coarse_iters=2)
+    graph, sc = _slide_sim(1, **over)
+    eager, _ = _slide_sim(1, **over)
+    kept, _ = _slide_sim(1, **over)
+    eager.use_graphs = False
+    for frame in range(1, 6):
+        if frame == 4:
+            graph.use_multigrid = eager.use_multigrid = False
+        for s in (graph, eager, kept):
+            s.set_fiber_activation(sc.activation(frame))
+            s.step_frame(frame)
+    a, b, c = (s.positions_np() for s in (graph, eager, kept))
+    assert np.isfinite(a).all()
+    assert np.abs(a - b).max() <= 1e-4  # the restriction's sums are float atomics
+    assert np.abs(a - c).max() > 1e-4

@@ -62,3 +62,18 @@ def test_frames_that_one_launch_does_not_take_go_substep_by_substep():
         e = _FrameEngine()
         assert XpbdEngine._fused_substeps(e, n_sub, n_iters, 0, 0, 0) is fits
         assert e.launched == ([(n_sub, n_iters)] * 2 if fits else [])
+
+
+def test_few_iterations_by_themselves_take_the_ring():
+    """The mailbox launch costs more to start than it saves on a few
+    iterations; whoever chose another kind of launch keeps it."""
+    from types import SimpleNamespace
+    for n_tets, n_tiles, first in ((28_046, 439, 2), (256 * 444, 444, 2), (256 * 444 + 1, 444, 10), (470_478, 444, 10)):
+        for sync in ("exchange", "grid", "neighbour"):
+            taken = []
+            e = SimpleNamespace(layout=SimpleNamespace(n_tets=n_tets, n_tiles=n_tiles), persistent_sync=sync,
+                                _ring_iterations=lambda n: taken.append("ring"),
+                                _fused_iterations=lambda n: taken.append("fused"))
+            for n in (1, first - 1, first, 20):
+                XpbdEngine._jacobi_iterations(e, n)
+            assert taken == (["ring", "ring", "fused", "fused"] if sync == "exchange" else ["fused"] * 4)
