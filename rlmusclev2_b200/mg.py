@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import operator
 import weakref
 from pathlib import Path
 
@@ -63,8 +64,8 @@ class _LaunchValues:
     """The values that a frame's launches take from the host objects ``parts``:
     their numbers, texts, tuples, tensors (by identity) and parameter structs.
     A captured frame holds them as they were; ``same`` says whether they still
-    are.  One comparison per attribute, 11 us for a simulator, where the
-    launches of an eager frame take milliseconds."""
+    are: while nothing is assigned, identities tell, without a Python
+    operation per attribute (the eager launches of a frame take milliseconds)."""
 
     #: attributes that change from frame to frame and that no launch reads
     BOOKKEEPING = frozenset({"step_cnt", "slide_interval", "_frame_loaded", "_reproject", "_status_pending",
@@ -78,22 +79,30 @@ class _LaunchValues:
             names = [k for k, v in d.items() if k not in self.BOOKKEEPING
                      and (v is None or isinstance(v, (int, float, str, tuple, np.generic, torch.Tensor)))]
             structs = [k for k, v in d.items() if isinstance(v, C.Structure)]
-            self.rows.append((weakref.ref(p), len(d), names, [d[k] for k in names], structs,
-                              [bytes(d[k]) for k in structs]))
+            names += structs
+            get = operator.itemgetter(*names, names[0]) if names else (lambda d: ())  # two names at least: a tuple
+            self.rows.append((weakref.ref(p), len(d), get, get(d), [(d[k], bytes(d[k])) for k in structs]))
 
     @staticmethod
     def _differ(a, b) -> bool:
-        return a is not b and (type(a) is not type(b) or isinstance(a, torch.Tensor) or bool(a != b))
+        return a is not b and (type(a) is not type(b) or isinstance(a, (torch.Tensor, C.Structure)) or bool(a != b))
 
     def same(self, parts: list) -> bool:
         if len(parts) != len(self.rows):
             return False
-        for p, (ref, n, names, values, structs, contents) in zip(parts, self.rows):
+        for p, (ref, n, get, values, structs) in zip(parts, self.rows):
             d = p.__dict__
-            if (ref() is not p or len(d) != n or any(map(self._differ, map(d.get, names), values))
-                    or any(not isinstance(d.get(k), C.Structure) or bytes(d[k]) != c
-                           for k, c in zip(structs, contents))):
+            if ref() is not p or len(d) != n:
                 return False
+            try:
+                now = get(d)
+            except KeyError:
+                return False
+            if not all(map(operator.is_, now, values)) and any(map(self._differ, now, values)):
+                return False
+            for s, content in structs:
+                if bytes(s) != content:
+                    return False
         return True
 
 
