@@ -4,6 +4,7 @@
 #include <stdio.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/xpbd_b200.h"
 #include "xpbd_common.cuh"
@@ -61,7 +62,6 @@ __global__ void k_blend_to_target(int n, const int* __restrict__ idx, int nv, fl
 }
 
 constexpr int kBrick = 8;      // 8^3 nodes per brick, a thread each
-constexpr int kRun = 4;        // bricks per CTA
 constexpr int kMaxCaps = 256;  // indices fit a byte
 
 struct CapW {
@@ -77,25 +77,39 @@ __device__ __forceinline__ float cap_phi(const CapW& c, float3 x) {
     return len(d) - c.r;
 }
 
-// One CTA per kRun 8x8x8 bricks of grid nodes along x: the capsules are posed
+// One CTA per RUN 8x8x8 bricks of grid nodes along x: the capsules are posed
 // once, each brick keeps only those whose distance to its centre is within band
 // + the brick's half diagonal, then every node takes the min over its brick's
 // short list (band elsewhere).
 //
 // The bytes written take 10 us for 256^3 nodes; the chain before them (capsule
 // loads, pose, distance, two barriers) is as long for one brick as for four and
-// bounded the kernel at 62 us for 256^3 (100 us for the 64 grids of a batch, whose
-// frame went from 1,336 to 1,269 us with four bricks a CTA).
+// bounds the kernel: four bricks a CTA where that leaves two CTAs for each of 148
+// SMs, else one, which fills more of them and has a fourth of the work in a row.
+// us in a graph with one and four bricks, 20 capsules: 2.7 and 4.5 for 32^3 nodes,
+// 3.1 and 3.6 for 64^3, 4.1 and 4.1 for 80^3 (the first with 300 CTAs of four), 9.3
+// and 6.3 for 128^3, 59 and 30 for 256^3; 89 and 35 for 64 grids of 64^3, 2 capsules.
+template <int RUN>
 struct BakeShared {
     CapW cap[kMaxCaps];
-    int n[kRun];
-    uint8_t list[kRun][kMaxCaps];
+    int n[RUN];
+    uint8_t list[RUN][kMaxCaps];  // not used with one brick: cap holds its capsules only
 };
 
+template <int RUN>
 __device__ __forceinline__ void bake_bricks(const XpbdSdf& S, int bx0, int by, int bz, int nc,
                                             const XpbdCapsule* __restrict__ caps, const float* __restrict__ tr,
-                                            float band, BakeShared& sm) {
-    if (threadIdx.x < kRun) sm.n[threadIdx.x] = 0;
+                                            float band, BakeShared<RUN>& sm) {
+    const float hb = 0.5f * S.h * float(kBrick - 1);
+    const float brad = hb * 1.7320508f;
+    auto near = [&](const CapW& w, int j) {
+        const float3 bc = make_float3(S.origin[0] + S.h * float((bx0 + j) * kBrick) + hb,
+                                      S.origin[1] + S.h * float(by * kBrick) + hb,
+                                      S.origin[2] + S.h * float(bz * kBrick) + hb);
+        return cap_phi(w, bc) <= band + brad;
+    };
+    if (threadIdx.x < RUN) sm.n[threadIdx.x] = 0;
+    if (RUN == 1) __syncthreads();
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
         const XpbdCapsule K = caps[c];
         float3 a = make_float3(K.center[0] - K.half * K.axis[0], K.center[1] - K.half * K.axis[1],
@@ -110,49 +124,52 @@ __device__ __forceinline__ void bake_bricks(const XpbdSdf& S, int bx0, int by, i
             b = make_float3(T[0] * b0.x + T[1] * b0.y + T[2] * b0.z + T[3], T[4] * b0.x + T[5] * b0.y + T[6] * b0.z + T[7],
                             T[8] * b0.x + T[9] * b0.y + T[10] * b0.z + T[11]);
         }
-        sm.cap[c] = CapW{a, b, K.radius};
+        const CapW w{a, b, K.radius};
+        if (RUN > 1)
+            sm.cap[c] = w;
+        else if (near(w, 0))
+            sm.cap[atomicAdd(&sm.n[0], 1)] = w;
     }
     __syncthreads();
-    const float hb = 0.5f * S.h * float(kBrick - 1);
-    const float brad = hb * 1.7320508f;
-    for (int k = threadIdx.x; k < nc * kRun; k += blockDim.x) {
-        const int c = k / kRun, j = k % kRun;
-        const float3 bc = make_float3(S.origin[0] + S.h * float((bx0 + j) * kBrick) + hb,
-                                      S.origin[1] + S.h * float(by * kBrick) + hb,
-                                      S.origin[2] + S.h * float(bz * kBrick) + hb);
-        if (cap_phi(sm.cap[c], bc) <= band + brad) sm.list[j][atomicAdd(&sm.n[j], 1)] = uint8_t(c);
+    if (RUN > 1) {
+        for (int k = threadIdx.x; k < nc * RUN; k += blockDim.x) {
+            const int c = k / RUN, j = k % RUN;
+            if (near(sm.cap[c], j)) sm.list[j][atomicAdd(&sm.n[j], 1)] = uint8_t(c);
+        }
+        __syncthreads();
     }
-    __syncthreads();
     const int lx = threadIdx.x & 7, ly = (threadIdx.x >> 3) & 7, lz = threadIdx.x >> 6;
     const int iy = by * kBrick + ly, iz = bz * kBrick + lz;
     if (iy >= S.ny || iz >= S.nz) return;
     float* row = const_cast<float*>(S.phi) + (size_t(iz) * S.ny + iy) * S.nx;
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) {
+    for (int j = 0; j < RUN; ++j) {
         const int ix = (bx0 + j) * kBrick + lx;
         if (ix >= S.nx) break;
         const float3 x = make_float3(S.origin[0] + S.h * float(ix), S.origin[1] + S.h * float(iy),
                                      S.origin[2] + S.h * float(iz));
         float phi = band;
         const int n = sm.n[j];
-        for (int k = 0; k < n; ++k) phi = fminf(phi, cap_phi(sm.cap[sm.list[j][k]], x));
+        for (int k = 0; k < n; ++k) phi = fminf(phi, cap_phi(sm.cap[RUN > 1 ? sm.list[j][k] : k], x));
         row[ix] = phi;
     }
 }
 
+template <int RUN>
 __global__ void __launch_bounds__(512) k_sdf_bake(const __grid_constant__ XpbdSdf S, int nc,
                                                   const XpbdCapsule* __restrict__ caps,
                                                   const float* __restrict__ tr, float band) {
-    __shared__ BakeShared sm;
-    bake_bricks(S, kRun * blockIdx.x, blockIdx.y, blockIdx.z, nc, caps, tr, band, sm);
+    __shared__ BakeShared<RUN> sm;
+    bake_bricks<RUN>(S, RUN * blockIdx.x, blockIdx.y, blockIdx.z, nc, caps, tr, band, sm);
 }
 
 // Batched: blockIdx.z runs over (instance, brick z); instance i bakes its own
 // grid from its own capsules caps[i * cpi .. (i + 1) * cpi).
+template <int RUN>
 __global__ void __launch_bounds__(512) k_sdf_bake_batched(const __grid_constant__ XpbdSdfBatch B, int cpi,
                                                           const XpbdCapsule* __restrict__ caps,
                                                           const float* __restrict__ tr, float band, int nbz) {
-    __shared__ BakeShared sm;
+    __shared__ BakeShared<RUN> sm;
     const int inst = blockIdx.z / nbz, bz = blockIdx.z % nbz;
     const float4 fr = reinterpret_cast<const float4*>(B.frame)[inst];
     XpbdSdf S;
@@ -167,8 +184,8 @@ __global__ void __launch_bounds__(512) k_sdf_bake_batched(const __grid_constant_
     S.contact_offset = B.contact_offset;
     S.max_push = B.max_push;
     S.reserved = 0;
-    bake_bricks(S, kRun * blockIdx.x, blockIdx.y, bz, cpi, caps + size_t(inst) * cpi,
-                tr ? tr + size_t(inst) * cpi * 12 : nullptr, band, sm);
+    bake_bricks<RUN>(S, RUN * blockIdx.x, blockIdx.y, bz, cpi, caps + size_t(inst) * cpi,
+                     tr ? tr + size_t(inst) * cpi * 12 : nullptr, band, sm);
 }
 
 __global__ void k_gather(int n, int width, const int32_t* __restrict__ idx, const float* __restrict__ src, int ss,
@@ -177,6 +194,18 @@ __global__ void k_gather(int n, int width, const int32_t* __restrict__ idx, cons
     if (i >= n) return;
     const int j = idx[i];
     for (int c = 0; c < width; ++c) dst[size_t(i) * ds + c] = src[size_t(j) * ss + c];
+}
+
+int bricks(int n) { return (n + kBrick - 1) / kBrick; }
+
+// Bricks per CTA of a bake over nx x ny nodes and nbz layers of bricks (see bake_bricks).
+template <class F>
+void with_run(int nx, int ny, int nbz, F f) {
+    const dim3 four((bricks(nx) + 3) / 4, bricks(ny), nbz);
+    if (int64_t(four.x) * four.y * four.z >= 2 * 148)
+        f(std::integral_constant<int, 4>{}, four);
+    else
+        f(std::integral_constant<int, 1>{}, dim3(bricks(nx), bricks(ny), nbz));
 }
 
 }  // namespace
@@ -217,8 +246,10 @@ int xpbd_sdf_bake_capsules(const XpbdSdf* sdf, int32_t n_caps, const XpbdCapsule
         return fail(XPBD_ERR_ARG, "xpbd_sdf_bake_capsules: bad grid");
     if (n_caps < 0 || n_caps > kMaxCaps || (n_caps > 0 && !caps))
         return fail(XPBD_ERR_LIMIT, "xpbd_sdf_bake_capsules: 0 <= n_caps <= 256 required");
-    dim3 grid((sdf->nx + kBrick * kRun - 1) / (kBrick * kRun), (sdf->ny + kBrick - 1) / kBrick, (sdf->nz + kBrick - 1) / kBrick);
-    k_sdf_bake<<<grid, kBrick * kBrick * kBrick, 0, (cudaStream_t)stream>>>(*sdf, n_caps, caps, transforms, band);
+    with_run(sdf->nx, sdf->ny, bricks(sdf->nz), [&](auto run, dim3 grid) {
+        k_sdf_bake<decltype(run)::value><<<grid, kBrick * kBrick * kBrick, 0, (cudaStream_t)stream>>>(
+            *sdf, n_caps, caps, transforms, band);
+    });
     return cuda_check("xpbd_sdf_bake_capsules");
 }
 
@@ -230,11 +261,12 @@ int xpbd_sdf_bake_capsules_batched(const XpbdSdfBatch* sdf, int32_t caps_per_ins
     if (!aligned16(sdf->frame)) return fail(XPBD_ERR_ALIGN, "xpbd_sdf_bake_capsules_batched: frame alignment");
     if (caps_per_inst < 0 || caps_per_inst > kMaxCaps || (caps_per_inst > 0 && !caps))
         return fail(XPBD_ERR_LIMIT, "xpbd_sdf_bake_capsules_batched: 0 <= caps_per_inst <= 256 required");
-    const int nbz = (sdf->nz + kBrick - 1) / kBrick;
+    const int nbz = bricks(sdf->nz);
     if (int64_t(nbz) * sdf->n_inst > 65535) return fail(XPBD_ERR_LIMIT, "xpbd_sdf_bake_capsules_batched: too many grids");
-    dim3 grid((sdf->nx + kBrick * kRun - 1) / (kBrick * kRun), (sdf->ny + kBrick - 1) / kBrick, nbz * sdf->n_inst);
-    k_sdf_bake_batched<<<grid, kBrick * kBrick * kBrick, 0, (cudaStream_t)stream>>>(*sdf, caps_per_inst, caps,
-                                                                                   transforms, band, nbz);
+    with_run(sdf->nx, sdf->ny, nbz * sdf->n_inst, [&](auto run, dim3 grid) {
+        k_sdf_bake_batched<decltype(run)::value><<<grid, kBrick * kBrick * kBrick, 0, (cudaStream_t)stream>>>(
+            *sdf, caps_per_inst, caps, transforms, band, nbz);
+    });
     return cuda_check("xpbd_sdf_bake_capsules_batched");
 }
 

@@ -189,3 +189,44 @@ def test_autotune_times_frames_and_restores_the_state(monkeypatch):
     sim.nsubsteps -= 1
     sim.step_frame_inputs(3)
     assert np.isfinite(sim.positions_np()).all()
+
+
+@pytest.mark.parametrize("dims", [(31, 150, 150), (32, 145, 151), (33, 160, 129), (65, 120, 160), (96, 96, 81)])
+@pytest.mark.parametrize("n_caps", [0, 3, 256])
+def test_sdf_bake_of_four_bricks_a_cta(dims, n_caps):
+    """The same edges in grids large enough for four bricks a CTA (small ones take one)."""
+    test_sdf_bake_runs_of_bricks(dims, n_caps)
+
+
+@pytest.mark.parametrize("n_inst", [1, 9, 40])
+def test_batched_bake_with_one_and_four_bricks(n_inst):
+    """The bake of several grids equals each grid's own, bit for bit, whichever
+    number of bricks their CTAs take (41 x 33 x 24 nodes: 30 CTAs of four a grid)."""
+    lib = capi.load()
+    rng = np.random.default_rng(n_inst)
+    nx, ny, nz = 41, 33, 24
+    caps = np.zeros((2 * n_inst, 8), np.float32)
+    caps[:, :3] = rng.random((2 * n_inst, 3)) * 0.4
+    caps[:, 3] = 0.05
+    ax = rng.normal(size=(2 * n_inst, 3))
+    caps[:, 4:7] = ax / np.linalg.norm(ax, axis=1, keepdims=True)
+    caps[:, 7] = 0.01
+    d_caps = torch.from_numpy(caps).cuda()
+    frame = torch.zeros((n_inst, 4), device="cuda")
+    frame[:, 3] = 0.01
+    phi = torch.full((n_inst, nz, ny, nx), -9.0, device="cuda")
+    one = torch.full((n_inst, nz, ny, nx), -7.0, device="cuda")
+    inst = torch.zeros(1, dtype=torch.int32, device="cuda")
+    b = capi.XpbdSdfBatch()
+    b.phi, b.frame, b.vert_inst = phi.data_ptr(), frame.data_ptr(), inst.data_ptr()
+    b.n_inst, b.nx, b.ny, b.nz = n_inst, nx, ny, nz
+    assert lib.xpbd_sdf_bake_capsules_batched(C.byref(b), 2, C.c_void_p(d_caps.data_ptr()), None, C.c_float(0.03),
+                                              None) == 0
+    for i in range(n_inst):
+        s = capi.XpbdSdf()
+        s.phi, s.nx, s.ny, s.nz, s.h = one[i].data_ptr(), nx, ny, nz, 0.01
+        assert lib.xpbd_sdf_bake_capsules(C.byref(s), 2, C.c_void_p(d_caps[2 * i:].data_ptr()), None, C.c_float(0.03),
+                                          None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(phi, one)
+    assert float(phi.min()) < 0.0 and float(phi.max()) <= 0.03 + 1e-9
